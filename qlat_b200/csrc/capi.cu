@@ -836,6 +836,12 @@ int library_stream(cudaStream_t* st)
   return QGB_OK;
 }
 
+// F = the gauge action's force at FP64 links U, both device buffers of lattice g (flowed.cu).
+int force_on(const Geo& g, const void* U, void* out, double beta, double c1)
+{
+  QGB_CTX();
+  return force<double>(g, FORCE_SET, fargs(U, out, beta, c1, 0.0));
+}
 // Lets the allocation-free entry point (noalloc.cu) report through qgb_last_error.
 void set_last_error(const std::string& msg) { g_err = msg; }
 // The library's reusable device buffers (zeroed when first allocated).

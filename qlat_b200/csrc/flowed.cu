@@ -15,17 +15,19 @@
 // force is propagated back through the steps (the transpose of each step's
 // Jacobian) with the force of the log-determinants added at each step.
 //
-// Layout: one thread per site.  The staple of the flowed links goes to a
-// color-matrix field of multiplicity 1; per flowed link, a per-step table
-// (exp(ad X), J(-ad X), the 8 traces of the determinant force and
-// (-eps) M'^-1 J(X)) feeds the per-site pass over the (link, flowed link)
-// pairs of the reference's set_xl_nu_from_mask_mu_yl_m.
+// A step is one launch over the flowed links (k_flow_step).  On the way back
+// that launch also forms, per flowed link, the one 3 x 3 matrix that carries
+// its part of the force and of the determinant's force to the links of its
+// staples, and a second launch over the links (k_flow_force_step) gathers it
+// over the pairs of the reference's set_xl_nu_from_mask_mu_yl_m.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
 
+#include <mutex>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/qlat_b200.h"
@@ -37,20 +39,16 @@ namespace qgb
 void set_last_error(const std::string& msg);
 void* field_data(const qgb_field* f);
 int library_stream(cudaStream_t* st);
+int force_on(const Geo& g, const void* U, void* out, double beta, double c1);
 }
 
 namespace
 {
 using namespace qgb;
 
-// ---- su(3) basis (matrix-hmc.h:76-124) and 8 x 8 real matrices -------------
+// ---- su(3) basis (matrix-hmc.h:76-124) and the adjoint representation -------
 
-struct A8 {
-  double m[64];  // row-major: (a, b) at m[8 a + b]
-};
-
-__constant__ double c_ts[8][18];  // T_a = make_anti_hermitian_matrix(e_a)
-__constant__ double c_f[8][64];   // f[c](a, b) = basis_c(T_a T_b - T_b T_a)
+constexpr double SQRT3 = 1.7320508075688772;
 
 __host__ __device__ inline M3<double> anti_herm_from_basis(const double* b)
 {
@@ -82,578 +80,501 @@ __host__ __device__ inline void basis_of(const M3<double>& m, double* b)
   b[7] = sqrt(3.0) * 0.5 * (m.e[0].im + m.e[4].im);
 }
 
-__device__ inline M3<double> ts(int a)
+// r = -ad_x v, the basis coefficients of [v, x] (T_a = i lambda_a, so [T_a, T_b] = -2 f_abc T_c and
+// r_c = 2 sum_ab f_abc x_a v_b): the nine independent structure constants of su(3), 54 multiply-adds
+// on registers instead of an 8 x 8 matrix-vector product.
+__host__ __device__ __forceinline__ void minus_ad(double (&r)[8], const double (&x)[8], const double (&v)[8])
 {
-  M3<double> t;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) t.e[k] = cx<double>(c_ts[a][2 * k], c_ts[a][2 * k + 1]);
-  return t;
+  for (int c = 0; c < 8; ++c) r[c] = 0.0;
+#define QGB_F(i, j, k, f)                                                              \
+  r[k - 1] = fma(f * x[i - 1], v[j - 1], fma(-(f * x[j - 1]), v[i - 1], r[k - 1]));    \
+  r[i - 1] = fma(f * x[j - 1], v[k - 1], fma(-(f * x[k - 1]), v[j - 1], r[i - 1]));    \
+  r[j - 1] = fma(f * x[k - 1], v[i - 1], fma(-(f * x[i - 1]), v[k - 1], r[j - 1]));
+  QGB_F(1, 2, 3, 2.0)
+  QGB_F(1, 4, 7, 1.0)
+  QGB_F(1, 5, 6, -1.0)
+  QGB_F(2, 4, 6, 1.0)
+  QGB_F(2, 5, 7, 1.0)
+  QGB_F(3, 4, 5, 1.0)
+  QGB_F(3, 6, 7, -1.0)
+  QGB_F(4, 5, 8, SQRT3)
+  QGB_F(6, 7, 8, SQRT3)
+#undef QGB_F
 }
 
-__device__ inline void a8_mul(A8& r, const A8& x, const A8& y)
+// ---- masks and lattice walks (flowed-hmc.cpp:71-110) ----------------------
+
+// Sites of mask 2 have an even sum of (x_k / size), those of mask 1 an odd one.
+// The i-th masked site, x fastest (extents are multiples of 2 size).
+template <int SZ>
+__device__ __forceinline__ Coord masked_site(const Geo& g, long i, int mask)
 {
-  for (int i = 0; i < 8; ++i)
-    for (int j = 0; j < 8; ++j) {
-      double s = 0.0;
-      for (int k = 0; k < 8; ++k) s += x.m[8 * i + k] * y.m[8 * k + j];
-      r.m[8 * i + j] = s;
+  const int hx = g.d[0] >> 1;
+  Coord x;
+  const int h = (int)(i % hx);
+  i /= hx;
+  x.c[1] = (int)(i % g.d[1]);
+  i /= g.d[1];
+  x.c[2] = (int)(i % g.d[2]);
+  x.c[3] = (int)(i / g.d[2]);
+  const int p = (x.c[1] / SZ + x.c[2] / SZ + x.c[3] / SZ + mask) & 1;
+  x.c[0] = SZ == 1 ? 2 * h + p : 4 * (h >> 1) + 2 * p + (h & 1);
+  return x;
+}
+
+// whether x + a mu + b nu (nu != mu) is in the mask; a, b >= -2
+template <int SZ>
+__device__ __forceinline__ bool in_mask(const Coord& x, int mu, int a, int nu, int b, int mask)
+{
+  int p = mask;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) p += (x.c[k] + (k == mu ? a : 0) + (k == nu ? b : 0) + 4) / SZ;
+  return (p & 1) == 0;
+}
+
+// The links of the staple path (e, [e,] mu, -e, [-e]) from x, e = s nu: link i's stored site and
+// direction; returns whether the path runs along it (else it enters as its adjoint).
+template <int SZ>
+__device__ __forceinline__ bool path_link(int i, int s, int& a, int& b, bool& along_mu)
+{
+  along_mu = i == SZ;
+  a = i > SZ ? 1 : 0;
+  if (i < SZ) {
+    b = s > 0 ? i : -i - 1;
+    return s > 0;
+  }
+  if (i == SZ) {
+    b = s * SZ;
+    return true;
+  }
+  const int j = 2 * SZ - i;  // links back: j = SZ - 1 .. 0
+  b = s > 0 ? j : -j - 1;
+  return s < 0;
+}
+
+// One staple of the link (x, mu): gf_plaq_staple_no_comm (qcd-acc.h:152-165) or
+// gf_srect_staple_no_comm (flowed-hmc.cpp:363-380), the path of direction s nu.
+template <int SZ>
+__device__ __forceinline__ M3<double> path_staple(const CField<double>& U, const Geo& g, const Coord& x, int mu, int nu,
+                                                  int s)
+{
+  M3<double> r = m3_unit<double>();
+#pragma unroll 1
+  for (int i = 0; i < 2 * SZ + 1; ++i) {
+    int a, b;
+    bool am;
+    const bool fwd = path_link<SZ>(i, s, a, b, am);
+    M3<double> l = U.ld(site_rt(g, x, mu, a, nu, b), am ? mu : nu);
+    if (!fwd) l = adj(l);
+    r = i == 0 ? l : mul(r, l);
+  }
+  return r;
+}
+
+// ---- kernels ----------------------------------------------------------------
+
+// What k_flow_step does with the masked links after forming their staples C.
+enum FlowMode {
+  FLOW_FORWARD = 0,   // U <- exp(-eps TA(U C^+)) U (flowed-hmc.cpp:424-454), the old links kept in `old`
+  FLOW_INVERSE = 1,   // the inverse, by fixed-point iterations (flowed-hmc.cpp:456-490)
+  FLOW_LN_DET = 2,    // FLOW_FORWARD, and ln det M' of each link
+  FLOW_PULL = 3,      // U <- old, then the link's part of the force's pull-back
+  FLOW_PULL_DET = 4   // the same with the force of the log-determinant
+};
+
+struct FlowArgs {
+  Geo g;
+  Cx<double>* U;
+  Cx<double>* old;  // the masked links of each site block, i fastest: old[(i / 32 * 9 + k) * 32 + i % 32]
+  int mask, mu;
+  double eps;
+  long n;  // masked links
+  int n_iter;
+  double* ln_det;         // FLOW_LN_DET: one value per masked link
+  const Cx<double>* Fin;  // FLOW_PULL*: the force after the step
+  Cx<double>* Fout;       // FLOW_PULL*: the force before it; the masked links' entries are written here
+  Cx<double>* Y;          // FLOW_PULL*: Z U of each masked link (k_flow_force_step), multiplicity 1
+};
+
+constexpr int FLOW_BS = 256, FLOW_LINKS = FLOW_BS / 8;
+constexpr int PAD = 66;  // doubles between two links' 8 x 8 matrices: the four links of a warp in distinct banks
+
+// y = A v for the 8 x 8 matrix at `a` (column-major)
+__device__ __forceinline__ void mat_vec(double (&y)[8], const double* a, const double (&v)[8])
+{
+#pragma unroll
+  for (int i = 0; i < 8; ++i) y[i] = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      const double2 t = *reinterpret_cast<const double2*>(a + 8 * k + i);
+      y[i] = fma(t.x, v[k], y[i]);
+      y[i + 1] = fma(t.y, v[k], y[i + 1]);
     }
 }
 
-__device__ inline void a8_scale(A8& r, double s, const A8& x)
+__device__ __forceinline__ void store_col(double* a, int b, const double (&v)[8])
 {
-  for (int i = 0; i < 64; ++i) r.m[i] = s * x.m[i];
+#pragma unroll
+  for (int i = 0; i < 8; i += 2) *reinterpret_cast<double2*>(a + 8 * b + i) = make_double2(v[i], v[i + 1]);
 }
 
-// make_adjoint_representation (matrix-hmc.h:294-306): sum_a (-basis_a(m)) f[a]
-__device__ inline void adjoint_rep(A8& am, const M3<double>& m)
+template <int N>
+__device__ __forceinline__ void sum8(double (&v)[N])  // over the 8 lanes of a link
 {
-  double b[8];
-  basis_of(m, b);
-  for (int i = 0; i < 64; ++i) am.m[i] = 0.0;
-  for (int a = 0; a < 8; ++a)
-    for (int i = 0; i < 64; ++i) am.m[i] += (-b[a]) * c_f[a][i];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
 }
 
-// make_matrix_exp (matrix-hmc.h:155-167) for 8 x 8: order-20 Horner
-__device__ inline void a8_exp(A8& r, const A8& a)
+__device__ __forceinline__ void sum8(M3<double>& m)
 {
-  A8 t2 = a, t3;
-  for (int j = 20; j > 1; --j) {
-    for (int i = 0; i < 64; ++i) t3.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) + (1.0 / j) * t2.m[i];
-    a8_mul(t2, a, t3);
-  }
-  for (int i = 0; i < 64; ++i) r.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) + t2.m[i];
-}
-
-// make_diff_exp_map (matrix-hmc.h:308-321): sum_k (-am)^k / (k+1)!, order 20
-__device__ inline void dexp_map(A8& r, const A8& am)
-{
-  A8 t2, t3;
-  for (int i = 0; i < 64; ++i) t2.m[i] = -am.m[i];
-  for (int j = 20; j > 1; --j) {
-    for (int i = 0; i < 64; ++i) t3.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) + (1.0 / (j + 1)) * t2.m[i];
-    A8 nam;
-    for (int i = 0; i < 64; ++i) nam.m[i] = -am.m[i];
-    a8_mul(t2, nam, t3);
-  }
-  for (int i = 0; i < 64; ++i) r.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) + 0.5 * t2.m[i];
-}
-
-// make_diff_exp_map_diff (matrix-hmc.h:341-362): derivative of dexp_map(am)
-// along f[a]
-__device__ inline void dexp_map_diff(A8& r, const A8& am, int a)
-{
-  A8 t2, dt2, t3, dt3, tmp1, tmp2;
-  for (int i = 0; i < 64; ++i) {
-    t2.m[i] = -am.m[i];
-    dt2.m[i] = c_f[a][i];
-  }
-  A8 fa;
-  for (int i = 0; i < 64; ++i) fa.m[i] = c_f[a][i];
-  for (int j = 20; j > 1; --j) {
-    for (int i = 0; i < 64; ++i) {
-      t3.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) + (1.0 / (j + 1)) * t2.m[i];
-      dt3.m[i] = (1.0 / (j + 1)) * dt2.m[i];
+#pragma unroll
+  for (int k = 0; k < 9; ++k)
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      m.e[k].re += __shfl_xor_sync(0xffffffffu, m.e[k].re, o);
+      m.e[k].im += __shfl_xor_sync(0xffffffffu, m.e[k].im, o);
     }
-    A8 nam;
-    for (int i = 0; i < 64; ++i) nam.m[i] = -am.m[i];
-    a8_mul(t2, nam, t3);
-    a8_mul(tmp1, fa, t3);
-    a8_mul(tmp2, am, dt3);
-    for (int i = 0; i < 64; ++i) dt2.m[i] = tmp1.m[i] - tmp2.m[i];
-  }
-  for (int i = 0; i < 64; ++i) r.m[i] = 0.5 * dt2.m[i];
 }
 
-// Determinant and inverse of an 8 x 8 matrix by Gaussian / Gauss-Jordan
-// elimination with partial pivoting, on local copies.  (The reference uses an
-// LU decomposition, matrix.h:275-420; the pivot order only changes rounding.)
-// Kept out of line: inlined into the large per-link kernel, an in-place LU
-// on the matrix struct gave a wrong determinant on this toolchain, while the
-// same code in a small kernel was right.
-__device__ __noinline__ double a8_det(const A8& m)
+// Inverse and determinant of the 8 x 8 matrix whose column b is lane b's `m` (Gauss-Jordan with
+// partial pivoting over the 8 lanes of a link; the pivot order of the reference's LU, matrix.h:275-420,
+// may differ, which changes only rounding).  inv: column b of the inverse.
+template <bool INV>
+__device__ __forceinline__ double gauss8(double (&m)[8], double (&inv)[8], int b)
 {
-  double a[64];
-  for (int i = 0; i < 64; ++i) a[i] = m.m[i];
   double det = 1.0;
+  if (INV) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) inv[i] = i == b ? 1.0 : 0.0;
+  }
+#pragma unroll
   for (int j = 0; j < 8; ++j) {
+    double col[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) col[i] = __shfl_sync(0xffffffffu, m[i], j, 8);
     int p = j;
-    double best = fabs(a[8 * j + j]);
-    for (int i = j + 1; i < 8; ++i) {
-      const double v = fabs(a[8 * i + j]);
-      if (v > best) {
-        best = v;
+    double best = fabs(col[j]);
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i)
+      if (fabs(col[i]) > best) {
+        best = fabs(col[i]);
         p = i;
       }
-    }
-    if (p != j) {
-      for (int k = 0; k < 8; ++k) {
-        const double t = a[8 * j + k];
-        a[8 * j + k] = a[8 * p + k];
-        a[8 * p + k] = t;
+    if (p != j) det = -det;
+#pragma unroll
+    for (int i = j + 1; i < 8; ++i)
+      if (i == p) {
+        double t = col[j];
+        col[j] = col[i];
+        col[i] = t;
+        t = m[j];
+        m[j] = m[i];
+        m[i] = t;
+        if (INV) {
+          t = inv[j];
+          inv[j] = inv[i];
+          inv[i] = t;
+        }
       }
-      det = -det;
-    }
-    const double piv = a[8 * j + j];
-    det *= piv;
-    if (piv == 0.0) return 0.0;
-    for (int i = j + 1; i < 8; ++i) {
-      const double f = a[8 * i + j] / piv;
-      for (int k = j + 1; k < 8; ++k) a[8 * i + k] -= f * a[8 * j + k];
+    det *= col[j];
+    // a zero pivot is a zero determinant (and no inverse)
+    const double r = !INV && col[j] == 0.0 ? 0.0 : 1.0 / col[j];
+    m[j] *= r;
+    if (INV) inv[j] *= r;
+#pragma unroll
+    for (int i = INV ? 0 : j + 1; i < 8; ++i) {
+      if (i == j) continue;
+      m[i] = fma(-col[i], m[j], m[i]);
+      if (INV) inv[i] = fma(-col[i], inv[j], inv[i]);
     }
   }
   return det;
 }
 
-__device__ __noinline__ void a8_inverse(A8& r, const A8& m)
+// One step of a flow, one launch.  Eight lanes per masked link, 32 links per block.
+//
+// The six staples of a link go to six of its lanes (a link's path is a chain of 2 or 4 dependent
+// products; one thread per link left 4096 links on 8^3 x 16 far short of filling the GPU) and are
+// added by shuffles.  No updated link enters another updated link's staple, so the update is in place.
+//
+// The 8 x 8 matrices of the Jacobian M' = 1 - eps J(X) N (flowed-hmc.cpp:926-955, 1011-1025,
+// 1117-1162) live one column per lane in registers.  With B = -ad X, applied by minus_ad:
+//   J(X) = sum_k B^k / (k+1)!  from the powers B^k e_b of each lane's own unit vector,
+//   the derivative of J along f[e] traced with W = eps^2 N M'^-1: tr(f[e] G),
+//     G = sum_k S_k / (k+1)!, S_{k+1} = B S_k + W B^k, S_1 = W, also column by column,
+// both the reference's order-20 polynomials, cut once the omitted terms are below 2^-58 of the sum.
+// One thread per link held all of it in local memory and differentiated J eight times over: 2.57 ms
+// a step on 8^3 x 16 (with the staple's own launch, 2.58), against 35 us (size 1) and 27 us (size 2) here.
+// At 4096 links it is bound by the latency of its chains (4 warps' worth of links per SM), not by FP64 rate.
+template <int SZ, int MODE>
+__global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
 {
-  double a[64], x[64];
-  for (int i = 0; i < 64; ++i) {
-    a[i] = m.m[i];
-    x[i] = (i % 9 == 0) ? 1.0 : 0.0;
+  constexpr bool PULL = MODE == FLOW_PULL || MODE == FLOW_PULL_DET;
+  constexpr bool DET = MODE == FLOW_LN_DET || MODE == FLOW_PULL_DET;
+  __shared__ __align__(16) double sA[DET ? FLOW_LINKS * PAD : 2], sB[DET ? FLOW_LINKS * PAD : 2];
+  __shared__ Cx<double> sC[PULL ? 1 : 9][FLOW_LINKS];
+  const int b = threadIdx.x & 7, w = threadIdx.x >> 3;
+  const long i0 = (long)blockIdx.x * FLOW_LINKS + w;
+  const long i = i0 < a.n ? i0 : a.n - 1;  // every lane stays for the shuffles
+  const Geo& g = a.g;
+  const int mu = a.mu;
+  const Coord x = masked_site<SZ>(g, i, a.mask);
+  const long s = site_rt(g, x, 0, 0, 1, 0);
+  const CField<double> U{a.U, g.V};
+  const WField<double> Uw{a.U, g.V};
+  M3<double> c = m3_zero<double>();
+  if (b < 6) c = path_staple<SZ>(U, g, x, mu, (mu + 1 + (b >> 1)) & 3, b & 1 ? -1 : 1);
+  sum8(c);
+  M3<double> u;
+  if (PULL) {
+    const Cx<double>* q = a.old + ((i >> 5) * 9) * 32 + (i & 31);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) u.e[k] = q[32 * k];
+    if (b == 0 && i0 < a.n) Uw.st(s, mu, u);  // nobody's staple of this step reads it
+  } else {
+    u = Uw.ld(s, mu);
   }
-  for (int j = 0; j < 8; ++j) {
-    int p = j;
-    double best = fabs(a[8 * j + j]);
-    for (int i = j + 1; i < 8; ++i) {
-      const double v = fabs(a[8 * i + j]);
-      if (v > best) {
-        best = v;
-        p = i;
+  if constexpr (DET || PULL) {
+    const M3<double> uc = mul_adj(u, c);
+    const M3<double> xm = scale(-a.eps, traceless_antiherm(uc));
+    double xb[8];
+    basis_of(xm, xb);
+    double nrm = 0.0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) nrm = fma(xb[k], xb[k], nrm);
+    nrm = 2.8284271247461903 * sqrt(nrm);  // |ad X| <= 2 |X| <= 2 sqrt(2) |x| (Frobenius)
+    double eb[8], q[8], jb[8], xp[8], t[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) q[k] = jb[k] = xp[k] = eb[k] = k == b ? 1.0 : 0.0;
+    // columns of J(X) and of exp(-ad X)
+    double bound = 1.0;
+#pragma unroll 1
+    for (int k = 1; k <= 20; ++k) {
+      const double inv = 1.0 / k, inv1 = 1.0 / (k + 1);
+      minus_ad(t, xb, q);
+#pragma unroll
+      for (int m = 0; m < 8; ++m) {
+        q[m] = t[m] * inv;
+        xp[m] += q[m];
+        jb[m] = fma(q[m], inv1, jb[m]);
       }
+      bound *= nrm * inv;
+      if (2.0 * bound * nrm < 3.4e-18 * (k + 1) && nrm < 0.5 * (k + 2)) break;
     }
-    if (p != j) {
-      for (int k = 0; k < 8; ++k) {
-        double t = a[8 * j + k];
-        a[8 * j + k] = a[8 * p + k];
-        a[8 * p + k] = t;
-        t = x[8 * j + k];
-        x[8 * j + k] = x[8 * p + k];
-        x[8 * p + k] = t;
-      }
-    }
-    const double inv = 1.0 / a[8 * j + j];
-    for (int k = 0; k < 8; ++k) {
-      a[8 * j + k] *= inv;
-      x[8 * j + k] *= inv;
-    }
-    for (int i = 0; i < 8; ++i) {
-      if (i == j) continue;
-      const double f = a[8 * i + j];
-      if (f == 0.0) continue;
-      for (int k = 0; k < 8; ++k) {
-        a[8 * i + k] -= f * a[8 * j + k];
-        x[8 * i + k] -= f * x[8 * j + k];
-      }
-    }
-  }
-  for (int i = 0; i < 64; ++i) r.m[i] = x[i];
-}
-
-// ---- masks and lattice walks (flowed-hmc.cpp:71-110) ----------------------
-
-struct C4 {
-  int x[4];
-};
-
-__device__ inline C4 shifted(C4 c, int dir)
-{
-  if (dir >= 0) c.x[dir] += 1;
-  else c.x[-dir - 1] -= 1;
-  return c;
-}
-
-__device__ inline bool same_coor(const C4& a, const C4& b)
-{
-  return a.x[0] == b.x[0] && a.x[1] == b.x[1] && a.x[2] == b.x[2] && a.x[3] == b.x[3];
-}
-
-__device__ inline int mask_of(const C4& c, int flow_size)
-{
-  if (flow_size == 1) return 2 - (c.x[0] + c.x[1] + c.x[2] + c.x[3] + 16 * 1024 * 1024) % 2;
-  return 2 - ((c.x[0] + 1024) / 2 + (c.x[1] + 1024) / 2 + (c.x[2] + 1024) / 2 + (c.x[3] + 1024) / 2) % 2;
-}
-
-__device__ inline long site_index(const Geo& g, const C4& c)
-{
-  long idx = 0;
-  for (int k = 3; k >= 0; --k) {
-    int v = c.x[k] % g.d[k];
-    if (v < 0) v += g.d[k];
-    idx = idx * g.d[k] + v;
-  }
-  return idx;
-}
-
-__device__ inline C4 coor_of_site(const Geo& g, long s)
-{
-  C4 c;
-  for (int k = 0; k < 4; ++k) {
-    c.x[k] = (int)(s % g.d[k]);
-    s /= g.d[k];
-  }
-  return c;
-}
-
-// gf_get_link: dir >= 0 is U_dir(x); dir < 0 is U_{-dir-1}(x - e)^+
-__device__ inline M3<double> get_link(const CField<double>& U, const Geo& g, const C4& x, int dir)
-{
-  if (dir >= 0) return U.ld(site_index(g, x), dir);
-  return adj(U.ld(site_index(g, shifted(x, dir)), -dir - 1));
-}
-
-// gf_wilson_line_no_comm (qcd-acc.h:23-41): ordered product from the unit matrix
-__device__ inline M3<double> wilson_line(const CField<double>& U, const Geo& g, C4 x, const int* path, int n)
-{
-  M3<double> r = m3_unit<double>();
-  for (int i = 0; i < n; ++i) {
-    r = mul(r, get_link(U, g, x, path[i]));
-    x = shifted(x, path[i]);
-  }
-  return r;
-}
-
-// gf_plaq_staple_no_comm (qcd-acc.h:152-165) / gf_srect_staple_no_comm (flowed-hmc.cpp:363-380)
-__device__ inline M3<double> flow_staple(const CField<double>& U, const Geo& g, const C4& x, int mu, int flow_size)
-{
-  M3<double> acc = m3_zero<double>();
-  for (int nu = -4; nu < 4; ++nu) {
-    if (nu == mu || -nu - 1 == mu) continue;
-    if (flow_size == 1) {
-      const int p[3] = {nu, mu, -nu - 1};
-      add_to(acc, wilson_line(U, g, x, p, 3));
-    } else {
-      const int p[5] = {nu, nu, mu, -nu - 1, -nu - 1};
-      add_to(acc, wilson_line(U, g, x, p, 5));
-    }
-  }
-  return acc;
-}
-
-__device__ inline int multiplicity_flow(bool same_mask, int flow_size)
-{
-  if (flow_size == 1) return same_mask ? 1 + 3 * 2 : 6 + 3 * 2;
-  return same_mask ? 1 + 3 * 4 : 6 + 3 * 4;
-}
-
-__device__ inline int mod4(int v) { return ((v % 4) + 4) % 4; }
-
-// set_xl_nu_from_mask_mu_yl_m (flowed-hmc.cpp:191-360): the m-th flowed link
-// (xl, mu) whose flow depends on the link (yl, nu)
-__device__ inline void pair_of(C4& xl, int& nu, int mask, int mu, const C4& yl, int m, int flow_size)
-{
-  const int mask_yl = mask_of(yl, flow_size);
-  if (flow_size == 1) {
-    if (mask == mask_yl) {
-      if (m < 1) {
-        nu = mu;
-        xl = yl;
+    double nb[8], mp[8], minv[8], ft[8];
+    M3<double> Q = m3_zero<double>();
+    if constexpr (DET) {
+      basis_of(traceless_antiherm(mul(anti_herm_from_basis(eb), uc)), nb);
+      double* A = sA + w * PAD;
+      double* Bm = sB + w * PAD;
+      store_col(A, b, jb);
+      store_col(Bm, b, nb);
+      __syncwarp();
+      mat_vec(t, A, nb);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) mp[k] = fma(-a.eps, t[k], eb[k]);
+      const double det = gauss8<MODE == FLOW_PULL_DET>(mp, minv, b);
+      if constexpr (MODE == FLOW_LN_DET) {
+        if (b == 0 && i0 < a.n) a.ln_det[i] = log(det);
       } else {
-        const int k = (m - 1) / 2, l = (m - 1) % 2;
-        nu = mod4(mu + k + 1);
-        xl = l == 0 ? yl : shifted(shifted(yl, nu), -mu - 1);
-      }
-    } else {
-      if (m < 6) {
-        nu = mu;
-        const int k = m / 2, l = m % 2;
-        const int dir = mod4(nu + k + 1);
-        xl = l == 0 ? shifted(yl, dir) : shifted(yl, -dir - 1);
-      } else {
-        const int k = (m - 6) / 2, l = (m - 6) % 2;
-        nu = mod4(mu + k + 1);
-        xl = l == 0 ? shifted(yl, -mu - 1) : shifted(yl, nu);
-      }
-    }
-    return;
-  }
-  const int nu_size = mask == mask_yl ? 1 : 6;
-  if (m < nu_size) {
-    nu = mu;
-    if (mask == mask_yl) {
-      xl = yl;
-    } else {
-      const int k = m / 2, l = m % 2;
-      const int dir = mod4(nu + k + 1);
-      xl = l == 0 ? shifted(shifted(yl, dir), dir) : shifted(shifted(yl, -dir - 1), -dir - 1);
-    }
-    return;
-  }
-  // set_xg_nu_from_mask_mu_yg_m_srect_nu_neq_mu
-  const int k = (m - nu_size) / 4, l = (m - nu_size) % 4;
-  nu = mod4(mu + k + 1);
-  C4 x;
-  int step;
-  if (l == 0) {
-    x = shifted(yl, -nu - 1);
-    step = nu;
-  } else if (l == 1) {
-    x = shifted(shifted(yl, nu), nu);
-    step = -nu - 1;
-  } else if (l == 2) {
-    x = shifted(shifted(yl, -mu - 1), -nu - 1);
-    step = nu;
-  } else {
-    x = shifted(shifted(shifted(yl, -mu - 1), nu), nu);
-    step = -nu - 1;
-  }
-  for (int it = 0; it < 8 && mask != mask_of(x, flow_size); ++it) x = shifted(x, step);
-  xl = x;
-}
-
-// is_same_link (flowed-hmc.cpp:71-83)
-__device__ inline int is_same_link(const C4& xl, int dir, const C4& yl, int nu)
-{
-  if (dir >= 0) return (dir == nu && same_coor(xl, yl)) ? 1 : 0;
-  return (-dir - 1 == nu && same_coor(shifted(xl, dir), yl)) ? -1 : 0;
-}
-
-// d_uc_mat_plaq_site_no_comm / d_uc_mat_srect_site_no_comm
-// (flowed-hmc.cpp:596-777): d TA(U C^+) / d(link (yl, nu)) = TA(uc_pre T uc_post)
-__device__ inline void d_uc_mat(M3<double>& uc_pre, M3<double>& uc_post, const CField<double>& C,
-                                const CField<double>& U, const Geo& g, const C4& xl, int mu, const C4& yl, int nu,
-                                int flow_size)
-{
-  const M3<double> u = U.ld(site_index(g, xl), mu);
-  if (mu == nu && same_coor(xl, yl)) {
-    uc_pre = m3_unit<double>();
-    uc_post = mul_adj(u, C.ld(site_index(g, xl), 0));
-    return;
-  }
-  // the staple path from xl: (dir1, [dir1,] mu, dir3, [dir3]) with dir1 = k, dir3 = -k-1
-  const int len = flow_size == 1 ? 3 : 5;
-  int path[5];
-  C4 pts[5];
-  int n_step = 0, is_pos = 0;
-  for (int k = -4; k < 4 && n_step == 0; ++k) {
-    if (flow_size == 1) {
-      path[0] = k;
-      path[1] = mu;
-      path[2] = -k - 1;
-    } else {
-      path[0] = k;
-      path[1] = k;
-      path[2] = mu;
-      path[3] = -k - 1;
-      path[4] = -k - 1;
-    }
-    pts[0] = xl;
-    for (int i = 1; i < len; ++i) pts[i] = shifted(pts[i - 1], path[i - 1]);
-    for (int i = 0; i < len; ++i) {
-      is_pos = is_same_link(pts[i], path[i], yl, nu);
-      if (is_pos != 0) {
-        n_step = i + 1;
-        break;
+        __syncwarp();
+        store_col(A, b, minv);
+        __syncwarp();
+        double wb[8], sb[8], gb[8], kb[8];
+        mat_vec(wb, Bm, minv);
+        mat_vec(kb, A, jb);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          wb[k] *= a.eps * a.eps;
+          kb[k] *= -a.eps;
+        }
+        __syncwarp();
+        store_col(Bm, b, wb);
+        __syncwarp();
+        // s_k = S_k / (k+1)! e_b and q_k = B^k / k! e_b
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          gb[k] = sb[k] = 0.5 * wb[k];
+          q[k] = eb[k];
+        }
+        bound = 1.0;
+#pragma unroll 1
+        for (int k = 1; k < 20; ++k) {
+          const double inv = 1.0 / k, i1 = 1.0 / (k + 1), i2 = 1.0 / (k + 2);
+          minus_ad(t, xb, q);
+#pragma unroll
+          for (int m = 0; m < 8; ++m) q[m] = t[m] * inv;
+          minus_ad(t, xb, sb);
+          double v[8];
+          mat_vec(v, Bm, q);
+#pragma unroll
+          for (int m = 0; m < 8; ++m) {
+            sb[m] = fma(t[m], i2, v[m] * (i1 * i2));
+            gb[m] += sb[m];
+          }
+          // |S_{k+1}| / (k+2)! <= (k+1) |B|^k |W| / (k+2)!
+          bound *= nrm * inv;
+          if (2.0 * bound * nrm < 3.4e-18 * (k + 1) && nrm < 0.5 * (k + 2)) break;
+        }
+        // e2dj[e] = tr(f[e] G) = -sum_b (2 f (e_b, G e_b))_e
+        minus_ad(ft, eb, gb);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ft[k] *= -0.5;
+        Q = scale(0.5, mul(anti_herm_from_basis(eb), anti_herm_from_basis(kb)));
       }
     }
-  }
-  // pre = links before the matching one, dl = the matching link, post = after
-  M3<double> pre = m3_unit<double>(), dl, post = m3_unit<double>();
-  bool pre_set = false, post_set = false;
-  for (int i = 0; i < len; ++i) {
-    const M3<double> l = get_link(U, g, pts[i], path[i]);
-    if (i + 1 < n_step) {
-      pre = pre_set ? mul(pre, l) : l;
-      pre_set = true;
-    } else if (i + 1 == n_step) {
-      dl = l;
-    } else {
-      post = post_set ? mul(post, l) : l;
-      post_set = true;
-    }
-  }
-  if (is_pos == 1) {
-    post = mul(dl, post);
-  } else {
-    pre = scale(-1.0, mul(pre, dl));  // - from the dagger of the link for T^b
-  }
-  uc_pre = scale(-1.0, mul_adj(u, post));  // - from C^+ for T^b
-  uc_post = adj(pre);
-}
-
-// n_mat from the pair's (uc_pre, uc_post): N(a, b) = basis_a(TA(uc_pre T_b uc_post))
-__device__ inline void n_mat(A8& n, const M3<double>& uc_pre, const M3<double>& uc_post)
-{
-  for (int b = 0; b < 8; ++b) {
-    const M3<double> d = traceless_antiherm(mul(mul(uc_pre, ts(b)), uc_post));
-    double v[8];
-    basis_of(d, v);
-    for (int a = 0; a < 8; ++a) n.m[8 * a + b] = v[a];
-  }
-}
-
-// ---- kernels ----------------------------------------------------------------
-
-__global__ void k_flow_staple(Geo g, const Cx<double>* Up, Cx<double>* Cp, int mask, int mu, int flow_size)
-{
-  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const C4 x = coor_of_site(g, s);
-  if (mask_of(x, flow_size) != mask) return;
-  const CField<double> U{Up, g.V};
-  WField<double>{Cp, g.V}.st(s, 0, flow_staple(U, g, x, mu, flow_size));
-}
-
-// gf_flow_plaq_mask_mu_no_comm (flowed-hmc.cpp:424-454) and its inverse
-// (456-490, n_iter fixed-point iterations)
-__global__ void k_flow_update(Geo g, Cx<double>* Up, const Cx<double>* Cp, int mask, int mu, int flow_size, double eps,
-                              int inverse, int n_iter)
-{
-  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const C4 x = coor_of_site(g, s);
-  if (mask_of(x, flow_size) != mask) return;
-  const WField<double> U{Up, g.V};
-  const M3<double> c = CField<double>{Cp, g.V}.ld(s, 0);
-  const M3<double> u1 = U.ld(s, mu);
-  M3<double> u0 = u1;
-  if (!inverse) {
-    const M3<double> z = scale(-1.0, traceless_antiherm(mul_adj(u1, c)));
-    M3<double> e = exp_ch(scale(eps, z));
-    unitarize(e);
-    u0 = mul(e, u1);
-  } else {
-    for (int n = 0; n < n_iter; ++n) {
-      const M3<double> xm = scale(-1.0, traceless_antiherm(mul_adj(u0, c)));
-      M3<double> e = exp_ch(scale(-eps, xm));
-      unitarize(e);
-      u0 = mul(e, u1);
-    }
-  }
-  U.st(s, mu, u0);
-}
-
-// Per flowed link: ln det M' (flowed-hmc.cpp:1011-1025, 1234-1255) into lnd[s]
-// and, for the force, the table T[s] = exp(ad X) | J(-ad X) | e2dj[8] |
-// (-eps) M'^-1 J(X) (flowed-hmc.cpp:926-955, 1117-1162).
-__global__ void k_flow_link_tables(Geo g, const Cx<double>* Up, const Cx<double>* Cp, int mask, int mu, int flow_size,
-                                   double eps, double* lnd, double* T)
-{
-  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const C4 x = coor_of_site(g, s);
-  if (mask_of(x, flow_size) != mask) {
-    if (lnd) lnd[s] = 0.0;
-    return;
-  }
-  const CField<double> U{Up, g.V};
-  const M3<double> u = U.ld(s, mu);
-  const M3<double> c = CField<double>{Cp, g.V}.ld(s, 0);
-  const M3<double> uc = mul_adj(u, c);
-  A8 n0;
-  for (int b = 0; b < 8; ++b) {
-    double v[8];
-    basis_of(traceless_antiherm(mul(mul(ts(b), u), adj(c))), v);
-    for (int a = 0; a < 8; ++a) n0.m[8 * a + b] = v[a];
-  }
-  const M3<double> xm = scale(-eps, traceless_antiherm(uc));
-  A8 adx, jx, ejx, mp;
-  adjoint_rep(adx, xm);
-  dexp_map(jx, adx);
-  a8_scale(ejx, eps, jx);
-  a8_mul(mp, ejx, n0);
-  for (int i = 0; i < 64; ++i) mp.m[i] = ((i % 9 == 0) ? 1.0 : 0.0) - mp.m[i];
-  if (lnd) lnd[s] = log(a8_det(mp));
-  if (!T) return;
-  double* t = T + s * 200;
-  // exp(ad X) and J(-ad X)
-  A8 tmp, nadx;
-  a8_exp(tmp, adx);
-  for (int i = 0; i < 64; ++i) t[i] = tmp.m[i];
-  for (int i = 0; i < 64; ++i) nadx.m[i] = -adx.m[i];
-  dexp_map(tmp, nadx);
-  for (int i = 0; i < 64; ++i) t[64 + i] = tmp.m[i];
-  // M'^-1
-  A8 inv;
-  a8_inverse(inv, mp);
-  // e2dj[e] = tr(dJ/dX_e  eps^2 N M'^-1)
-  A8 e2n, e2nmi;
-  a8_scale(e2n, eps * eps, n0);
-  a8_mul(e2nmi, e2n, inv);
-  for (int e = 0; e < 8; ++e) {
-    dexp_map_diff(tmp, adx, e);
-    double tr = 0.0;
-    for (int i = 0; i < 8; ++i)
-      for (int j = 0; j < 8; ++j) tr += tmp.m[8 * i + j] * e2nmi.m[8 * j + i];
-    t[128 + e] = tr;
-  }
-  // (-eps) M'^-1 J(X)
-  A8 einv;
-  a8_scale(einv, -eps, inv);
-  a8_mul(tmp, einv, jx);
-  for (int i = 0; i < 64; ++i) t[136 + i] = tmp.m[i];
-}
-
-// One step of the force propagation (flowed-hmc.cpp:1059-1091, 1164-1232,
-// 1366-1427): Fout(yl, nu) = sum over pairs of the transposed Jacobian
-// applied to Fin(xl, mu), plus Fin(yl, nu) for the links the step does not
-// move, plus the force of the step's log-determinants.
-__global__ void k_flow_force_step(Geo g, const Cx<double>* Up, const Cx<double>* Cp, const double* T,
-                                  const Cx<double>* Finp, Cx<double>* Foutp, int mask, int mu, int flow_size,
-                                  double eps, int with_det)
-{
-  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= g.V) return;
-  const C4 yl = coor_of_site(g, s);
-  const int mask_yl = mask_of(yl, flow_size);
-  const CField<double> U{Up, g.V}, C{Cp, g.V}, Fin{Finp, g.V};
-  M3<double> fprop[4], fdet[4];
-  for (int nu = 0; nu < 4; ++nu) fprop[nu] = fdet[nu] = m3_zero<double>();
-  const int nm = multiplicity_flow(mask == mask_yl, flow_size);
-  for (int m = 0; m < nm; ++m) {
-    C4 xl;
-    int nu;
-    pair_of(xl, nu, mask, mu, yl, m, flow_size);
-    M3<double> uc_pre, uc_post;
-    d_uc_mat(uc_pre, uc_post, C, U, g, xl, mu, yl, nu, flow_size);
-    A8 n;
-    n_mat(n, uc_pre, uc_post);
-    const double* t = T + site_index(g, xl) * 200;
-    // m_mat = [exp(ad X) if the same link] - (eps J(-ad X)) N
-    A8 ej, mm;
-    for (int i = 0; i < 64; ++i) ej.m[i] = eps * t[64 + i];
-    a8_mul(mm, ej, n);
-    const bool same = mu == nu && same_coor(xl, yl);
-    for (int i = 0; i < 64; ++i) mm.m[i] = same ? t[i] - mm.m[i] : -mm.m[i];
-    double bb[8], ba[8];
-    basis_of(Fin.ld(site_index(g, xl), mu), bb);
-    for (int a = 0; a < 8; ++a) ba[a] = 0.0;
-    for (int b = 0; b < 8; ++b)
-      for (int a = 0; a < 8; ++a) ba[a] += bb[b] * mm.m[8 * b + a];
-    add_to(fprop[nu], anti_herm_from_basis(ba));
-    if (with_det) {
-      double fd[8];
-      for (int a = 0; a < 8; ++a) {
-        fd[a] = 0.0;
-        for (int e = 0; e < 8; ++e) fd[a] += n.m[8 * e + a] * t[128 + e];
-        const M3<double> ucm = mul(mul(uc_pre, ts(a)), uc_post);
-        for (int c = 0; c < 8; ++c) {
-          double dnb[8];
-          basis_of(traceless_antiherm(mul(ts(c), ucm)), dnb);
-          for (int b = 0; b < 8; ++b) fd[a] += t[136 + 8 * c + b] * dnb[b];
+    if constexpr (PULL) {
+      // Z = -W + (E + Q) / 2: W = eps (J(X) F) . T, E = e2dj . T, Q = sum_cb K_cb T_b T_c with K = -eps M'^-1 J(X)
+      double fb[8];
+      basis_of(CField<double>{a.Fin, g.V}.ld(s, mu), fb);
+      double fbb = 0.0;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) fbb = k == b ? fb[k] : fbb;
+      double z[8], r[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        z[k] = -a.eps * jb[k] * fbb;
+        if (DET) z[k] += ft[k];
+        r[k] = xp[k] * fbb;
+      }
+      sum8(z);
+      sum8(r);
+      M3<double> Z = anti_herm_from_basis(z);
+      if constexpr (DET) {
+        sum8(Q);
+        add_to(Z, Q);
+      }
+      // the link's own entry: Ad_{exp(-X)} F + TA(U C^+ Z); Y = Z U for the links of its staples
+      if (i0 < a.n) {
+        if (b == 0) WField<double>{a.Y, g.V}.st(s, 0, mul(Z, u));
+        if (b == 1) {
+          M3<double> f = anti_herm_from_basis(r);
+          add_to(f, traceless_antiherm(mul(uc, Z)));
+          WField<double>{a.Fout, g.V}.st(s, mu, f);
         }
       }
-      add_to(fdet[nu], scale(0.5, anti_herm_from_basis(fd)));
     }
   }
-  const WField<double> Fout{Foutp, g.V};
-  for (int nu = 0; nu < 4; ++nu) {
-    if (!(mask_yl == mask && mu == nu)) add_to(fprop[nu], Fin.ld(s, nu));
-    add_to(fprop[nu], fdet[nu]);
-    Fout.st(s, nu, fprop[nu]);
+  if constexpr (!PULL) {
+    // the block's links, one per lane of its first warp
+    if (b == 0) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) sC[k][w] = c.e[k];
+    }
+    __syncthreads();
+    if (threadIdx.x >= FLOW_LINKS) return;
+    const long j = (long)blockIdx.x * FLOW_LINKS + threadIdx.x;
+    if (j >= a.n) return;
+    const Coord xj = masked_site<SZ>(g, j, a.mask);
+    const long sj = site_rt(g, xj, 0, 0, 1, 0);
+    M3<double> cj;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) cj.e[k] = sC[k][threadIdx.x];
+    const M3<double> u1 = Uw.ld(sj, mu);
+    if (a.old != nullptr) {
+      Cx<double>* q = a.old + ((j >> 5) * 9) * 32 + (j & 31);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) q[32 * k] = u1.e[k];
+    }
+    M3<double> u0 = u1;
+    const double e = MODE == FLOW_INVERSE ? a.eps : -a.eps;
+#pragma unroll 1
+    for (int it = 0; it < (MODE == FLOW_INVERSE ? a.n_iter : 1); ++it) {
+      M3<double> ex = exp_su3(scale(e, traceless_antiherm(mul_adj(u0, cj))));
+      unitarize(ex);
+      u0 = mul(ex, u1);
+    }
+    Uw.st(sj, mu, u0);
   }
 }
 
-__global__ void k_sum_sites(long V, const double* v, double* out)
+// The part of the force's pull-back that reaches the link (y, nu) through a staple (flowed-hmc.cpp:596-777,
+// 1059-1091, 1164-1232, 1366-1427): a masked link (x, mu) whose staple path l_1 ... l_n holds (y, nu) as
+// its n-th link gives TA(uc_post Z uc_pre), which with Y = Z U is
+//   -(l_1 .. l_{n-1})^+ Y (l_n .. )^+ for a link the path runs along, +(l_1 .. l_n)^+ Y (l_{n+1} ..)^+ else.
+// (In the su(3) basis this is the sum over a of w_a n_mat(a, .) of the reference, with basis_a(TA(M)) =
+// -tr(T_a M)/2 moving the two factors around the trace.)  x = y + a mu + b nu in the staple's plane.
+template <int SZ>
+__device__ __forceinline__ void pull_path(M3<double>& acc, const CField<double>& U, const CField<double>& Y,
+                                          const Geo& g, const Coord& y, int mu, int nu, int a0, int b0, int s, int n)
 {
-  // one block: fixed-order sum of the per-site values
-  __shared__ double sm[256];
-  double t = 0.0;
-  for (long i = threadIdx.x; i < V; i += blockDim.x) t += v[i];
-  sm[threadIdx.x] = t;
+  M3<double> m = Y.ld(site_rt(g, y, mu, a0, nu, b0), 0);
+  int a, b;
+  bool am;
+  const bool along = path_link<SZ>(n, s, a, b, am);
+  const int cut = along ? n : n + 1;
+  auto link = [&](int i) {  // l_i^+
+    const bool fwd = path_link<SZ>(i, s, a, b, am);
+    M3<double> l = U.ld(site_rt(g, y, mu, a0 + a, nu, b0 + b), am ? mu : nu);
+    return fwd ? adj(l) : l;
+  };
+#pragma unroll 1
+  for (int i = 0; i < cut; ++i) m = mul(link(i), m);
+#pragma unroll 1
+  for (int i = 2 * SZ; i >= cut; --i) m = mul(m, link(i));
+  axpy(acc, along ? -1.0 : 1.0, m);
+}
+
+// Fout at every link but the masked ones (k_flow_step writes those): Fin plus what the staples pull back.
+// One thread per link; the pairs of set_xl_nu_from_mask_mu_yl_m (flowed-hmc.cpp:191-360) as the two masked
+// sites among the 2 SZ positions each side of the link allows.  2 SZ + 1 products of 3 x 3 matrices per
+// pair, no 8 x 8 ones: 761 us a step on 8^3 x 16 before, 16 us (size 1) and 34 us (size 2) now.
+template <int SZ>
+__global__ void __launch_bounds__(128) k_flow_force_step(Geo g, const Cx<double>* Up, const Cx<double>* Yp,
+                                                         const Cx<double>* Finp, Cx<double>* Foutp, int mask, int mu)
+{
+  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (s >= g.V) return;
+  const int nu = blockIdx.y;
+  const Coord y = coord_of(g, s);
+  const CField<double> U{Up, g.V}, Y{Yp, g.V};
+  M3<double> acc = m3_zero<double>();
+  if (nu == mu) {
+    if (in_mask<SZ>(y, 0, 0, 1, 0, mask)) return;
+#pragma unroll 1
+    for (int k = 0; k < 6; ++k) {
+      const int d = (mu + 1 + (k >> 1)) & 3, e = k & 1 ? -1 : 1;
+      pull_path<SZ>(acc, U, Y, g, y, mu, d, 0, -SZ * e, e, SZ);
+    }
+  } else {
+#pragma unroll 1
+    for (int side = 0; side < 2; ++side) {
+      // the path leaves along (links 0 .. SZ - 1, from x) or returns to (links SZ + 1 .. 2 SZ, at x + mu) this link
+      int left = SZ;
+#pragma unroll 1
+      for (int d = 1 - SZ; d <= SZ && left > 0; ++d) {
+        if (!in_mask<SZ>(y, mu, -side, nu, d, mask)) continue;
+        --left;
+        const int s2 = d <= 0 ? 1 : -1;
+        const int r = d <= 0 ? -d : d - 1;  // links between x and this one
+        pull_path<SZ>(acc, U, Y, g, y, mu, nu, -side, d, s2, side == 0 ? r : 2 * SZ - r);
+      }
+    }
+  }
+  M3<double> f = traceless_antiherm(acc);
+  add_to(f, CField<double>{Finp, g.V}.ld(s, nu));
+  WField<double>{Foutp, g.V}.st(s, nu, f);
+}
+
+__global__ void __launch_bounds__(1024) k_sum_links(long n, const double* v, double* out)
+{
+  // one block per step: fixed-order sum of its links' values
+  v += (size_t)blockIdx.x * n;
+  out += blockIdx.x;
+  __shared__ double sm[1024];
+  double t[4] = {0.0, 0.0, 0.0, 0.0};
+  for (long i = threadIdx.x; i < n; i += 4096)
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (i + 1024 * k < n) t[k] += v[i + 1024 * k];
+  sm[threadIdx.x] = (t[0] + t[1]) + (t[2] + t[3]);
   __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
+  for (int w = 512; w > 0; w >>= 1) {
     if ((int)threadIdx.x < w) sm[threadIdx.x] += sm[threadIdx.x + w];
     __syncthreads();
   }
@@ -679,51 +600,13 @@ int ffail(int code, const std::string& m)
     if (r_ != QGB_OK) return r_; \
   } while (0)
 
-int init_constants_here()
-{
-  static uint64_t done = 0;  // one bit per device
-  int dev = 0;
-  FL_CUDA(cudaGetDevice(&dev));
-  if (dev < 64 && (done >> dev) & 1u) return QGB_OK;
-  double tsh[8][18], fh[8][64];
-  M3<double> t[8];
-  for (int a = 0; a < 8; ++a) {
-    double b[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    b[a] = 1.0;
-    t[a] = anti_herm_from_basis(b);
-    for (int k = 0; k < 9; ++k) {
-      tsh[a][2 * k] = t[a].e[k].re;
-      tsh[a][2 * k + 1] = t[a].e[k].im;
-    }
-  }
-  for (int a = 0; a < 8; ++a)
-    for (int b = 0; b < 8; ++b) {
-      M3<double> ab = mul(t[a], t[b]), ba = mul(t[b], t[a]);
-      for (int k = 0; k < 9; ++k) {
-        ab.e[k].re -= ba.e[k].re;
-        ab.e[k].im -= ba.e[k].im;
-      }
-      double v[8];
-      basis_of(ab, v);
-      for (int c = 0; c < 8; ++c) fh[c][8 * a + b] = v[c];
-    }
-  FL_CUDA(cudaMemcpyToSymbol(c_ts, tsh, sizeof(tsh)));
-  FL_CUDA(cudaMemcpyToSymbol(c_f, fh, sizeof(fh)));
-  // the per-link 8 x 8 algebra keeps several KB of matrices per thread (a
-  // setting of this process's context only)
-  size_t stack = 0;
-  FL_CUDA(cudaDeviceGetLimit(&stack, cudaLimitStackSize));
-  if (stack < 16384) FL_CUDA(cudaDeviceSetLimit(cudaLimitStackSize, 16384));
-  if (dev < 64) done |= (uint64_t)1 << dev;
-  return QGB_OK;
-}
-
 struct FlowCtx {
   Geo g;
   cudaStream_t st = nullptr;
   long V = 0;
-  size_t bytes = 0;  // one gauge field
-  int blocks = 0;
+  size_t bytes = 0;      // one gauge field
+  long links = 0;        // links that one step moves
+  size_t old_bytes = 0;  // those links of one step, kept (FlowArgs::old)
 };
 
 int check_steps(const Geo& g, const qgb_flow_step* steps, int n)
@@ -740,22 +623,51 @@ int check_steps(const Geo& g, const qgb_flow_step* steps, int n)
   return QGB_OK;
 }
 
-// One flow step (or its inverse) in place on U (device buffer), C a scratch
-// color-matrix buffer of multiplicity 1.
-int flow_step_dev(const FlowCtx& c, void* U, void* C, const qgb_flow_step& f, bool inverse)
+// Work buffers of one call, in stream order.  The pool keeps at most 1 GiB from call to call (beyond that the
+// memory goes back to the device when the stream is next synchronised), and every call owns its buffers, so
+// calls of several threads do not share them.
+int work_pool(cudaMemPool_t* out)
 {
-  k_flow_staple<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)U, (Cx<double>*)C, f.mask, f.mu, f.flow_size);
-  FL_CUDA(cudaGetLastError());
-  k_flow_update<<<c.blocks, 128, 0, c.st>>>(c.g, (Cx<double>*)U, (const Cx<double>*)C, f.mask, f.mu, f.flow_size,
-                                            f.epsilon, inverse ? 1 : 0, 50);
-  FL_CUDA(cudaGetLastError());
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  FL_CUDA(cudaGetDevice(&dev));
+  if (dev >= 64) return ffail(QGB_ERR_CUDA, "flowed: device number out of range");
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    FL_CUDA(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = (uint64_t)1 << 30;
+    FL_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools[dev] = p;
+  }
+  *out = pools[dev];
   return QGB_OK;
 }
 
 struct DevBuf {
   void* p = nullptr;
-  ~DevBuf() { cudaFree(p); }
-  cudaError_t alloc(size_t b) { return cudaMalloc(&p, b); }
+  cudaStream_t st = nullptr;
+  DevBuf() = default;
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  ~DevBuf()
+  {
+    if (p) cudaFreeAsync(p, st);
+  }
+  int alloc(size_t b, cudaStream_t stream)
+  {
+    cudaMemPool_t pool = nullptr;
+    FL_RC(work_pool(&pool));
+    st = stream;
+    FL_CUDA(cudaMallocFromPoolAsync(&p, b > 0 ? b : 1, pool, stream));
+    return QGB_OK;
+  }
 };
 
 int setup(FlowCtx& c, const qgb_field* gf, int32_t n, const qgb_flow_step* steps)
@@ -768,10 +680,42 @@ int setup(FlowCtx& c, const qgb_field* gf, int32_t n, const qgb_flow_step* steps
   c.g.V = (long)ts[0] * ts[1] * ts[2] * ts[3];
   c.V = c.g.V;
   c.bytes = (size_t)padded_sites(c.V) * 72 * sizeof(double);
-  c.blocks = (int)((c.V + 127) / 128);
+  c.links = c.V / 2;
+  c.old_bytes = (size_t)padded_sites(c.links) * 18 * sizeof(double);
   FL_RC(qgb::library_stream(&c.st));
-  FL_RC(check_steps(c.g, steps, n));
-  return init_constants_here();
+  return check_steps(c.g, steps, n);
+}
+
+int check_output(const qgb_field* gf)
+{
+  int32_t prec = 0;
+  FL_RC(qgb_field_info(gf, nullptr, nullptr, nullptr, &prec));
+  if (prec != QGB_F64) return ffail(QGB_ERR_MISMATCH, "flowed: the flowed gauge field must be FP64");
+  return QGB_OK;
+}
+
+FlowArgs flow_args(const FlowCtx& c, void* U, const qgb_flow_step& f)
+{
+  FlowArgs a;
+  memset((void*)&a, 0, sizeof(a));
+  a.g = c.g;
+  a.U = (Cx<double>*)U;
+  a.mask = f.mask;
+  a.mu = f.mu;
+  a.eps = f.epsilon;
+  a.n = c.links;
+  a.n_iter = 50;
+  return a;
+}
+
+template <int MODE>
+int launch_flow_step(const FlowCtx& c, const FlowArgs& a, int flow_size)
+{
+  const unsigned grid = (unsigned)((c.links + FLOW_LINKS - 1) / FLOW_LINKS);
+  if (flow_size == 1) k_flow_step<1, MODE><<<grid, FLOW_BS, 0, c.st>>>(a);
+  else k_flow_step<2, MODE><<<grid, FLOW_BS, 0, c.st>>>(a);
+  FL_CUDA(cudaGetLastError());
+  return QGB_OK;
 }
 
 }  // namespace
@@ -839,12 +783,10 @@ int qgb_gf_flow(qgb_field* gf, const qgb_field* gf0, const qgb_flow_step* steps,
 {
   FlowCtx c;
   FL_RC(setup(c, gf0, n, steps));
+  FL_RC(check_output(gf));
   FL_RC(qgb_field_copy(gf, gf0));
-  DevBuf C;
-  FL_CUDA(C.alloc(c.bytes / 4));
   void* U = qgb::field_data(gf);
-  for (int i = 0; i < n; ++i) FL_RC(flow_step_dev(c, U, C.p, steps[i], false));
-  FL_CUDA(cudaStreamSynchronize(c.st));
+  for (int i = 0; i < n; ++i) FL_RC(launch_flow_step<FLOW_FORWARD>(c, flow_args(c, U, steps[i]), steps[i].flow_size));
   return QGB_OK;
 }
 
@@ -852,12 +794,11 @@ int qgb_gf_flow_inv(qgb_field* gf, const qgb_field* gf1, const qgb_flow_step* st
 {
   FlowCtx c;
   FL_RC(setup(c, gf1, n, steps));
+  FL_RC(check_output(gf));
   FL_RC(qgb_field_copy(gf, gf1));
-  DevBuf C;
-  FL_CUDA(C.alloc(c.bytes / 4));
   void* U = qgb::field_data(gf);
-  for (int i = n - 1; i >= 0; --i) FL_RC(flow_step_dev(c, U, C.p, steps[i], true));
-  FL_CUDA(cudaStreamSynchronize(c.st));
+  for (int i = n - 1; i >= 0; --i)
+    FL_RC(launch_flow_step<FLOW_INVERSE>(c, flow_args(c, U, steps[i]), steps[i].flow_size));
   return QGB_OK;
 }
 
@@ -867,28 +808,23 @@ int qgb_gf_flow_and_ln_det_node(qgb_field* gf, const qgb_field* gf0, const qgb_f
   FlowCtx c;
   FL_RC(setup(c, gf0, n, steps));
   if (!ln_det) return ffail(QGB_ERR_INVALID_ARG, "qgb_gf_flow_and_ln_det_node: null output");
+  FL_RC(check_output(gf));
   FL_RC(qgb_field_copy(gf, gf0));
-  DevBuf C, L, S;
-  FL_CUDA(C.alloc(c.bytes / 4));
-  FL_CUDA(L.alloc(c.V * sizeof(double)));
-  FL_CUDA(S.alloc((size_t)(n > 0 ? n : 1) * sizeof(double)));
+  DevBuf L, S;
+  FL_RC(L.alloc((size_t)c.links * sizeof(double) * (n > 0 ? n : 1), c.st));
+  FL_RC(S.alloc((size_t)(n > 0 ? n : 1) * sizeof(double), c.st));
   void* U = qgb::field_data(gf);
   for (int i = 0; i < n; ++i) {
-    const qgb_flow_step& f = steps[i];
-    k_flow_staple<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)U, (Cx<double>*)C.p, f.mask, f.mu,
-                                              f.flow_size);
-    FL_CUDA(cudaGetLastError());
-    k_flow_link_tables<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)U, (const Cx<double>*)C.p, f.mask, f.mu,
-                                                   f.flow_size, f.epsilon, (double*)L.p, nullptr);
-    FL_CUDA(cudaGetLastError());
-    k_sum_sites<<<1, 256, 0, c.st>>>(c.V, (const double*)L.p, (double*)S.p + i);
-    FL_CUDA(cudaGetLastError());
-    k_flow_update<<<c.blocks, 128, 0, c.st>>>(c.g, (Cx<double>*)U, (const Cx<double>*)C.p, f.mask, f.mu, f.flow_size,
-                                              f.epsilon, 0, 0);
-    FL_CUDA(cudaGetLastError());
+    FlowArgs a = flow_args(c, U, steps[i]);
+    a.ln_det = (double*)L.p + (size_t)i * c.links;
+    FL_RC(launch_flow_step<FLOW_LN_DET>(c, a, steps[i].flow_size));
   }
   std::vector<double> sums((size_t)(n > 0 ? n : 1), 0.0);
-  if (n > 0) FL_CUDA(cudaMemcpyAsync(sums.data(), S.p, n * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  if (n > 0) {
+    k_sum_links<<<n, 1024, 0, c.st>>>(c.links, (const double*)L.p, (double*)S.p);
+    FL_CUDA(cudaGetLastError());
+    FL_CUDA(cudaMemcpyAsync(sums.data(), S.p, n * sizeof(double), cudaMemcpyDeviceToHost, c.st));
+  }
   FL_CUDA(cudaStreamSynchronize(c.st));
   double t = 0.0;
   for (int i = 0; i < n; ++i) t += sums[i];
@@ -925,49 +861,48 @@ int flowed_force(qgb_field* gm_force, const qgb_field* gf0, const qgb_field* pre
 {
   FlowCtx c;
   FL_RC(setup(c, gf0, n, steps));
-  int32_t ts[4];
-  FL_RC(qgb_field_info(gf0, ts, nullptr, nullptr, nullptr));
-  // gf_ext_vec: the field before each step, then the flowed field
-  std::vector<DevBuf> G(n + 1);
-  for (int i = 0; i <= n; ++i) FL_CUDA(G[i].alloc(c.bytes));
-  DevBuf C, T, F2;
-  FL_CUDA(C.alloc(c.bytes / 4));
-  FL_CUDA(T.alloc((size_t)c.V * 200 * sizeof(double)));
-  FL_CUDA(F2.alloc(c.bytes));
-  FL_CUDA(cudaMemcpyAsync(G[0].p, qgb::field_data(gf0), c.bytes,
-                          cudaMemcpyDeviceToDevice, c.st));
+  int32_t ts[4], mult = 0, kind = 0, prec = 0;
+  FL_RC(qgb_field_info(gm_force, ts, &mult, &kind, &prec));
+  if (kind != QGB_KIND_COLOR_MATRIX || mult != 4 || prec != QGB_F64 || ts[0] != c.g.d[0] || ts[1] != c.g.d[1] ||
+      ts[2] != c.g.d[2] || ts[3] != c.g.d[3])
+    return ffail(QGB_ERR_MISMATCH, "flowed: the force must be an FP64 color-matrix field of multiplicity 4 on the "
+                                   "gauge field's lattice");
+  // one work field: the flow runs in it and keeps the links that each step replaces (an eighth of the field), and
+  // the way back puts them in place again
+  DevBuf G, old, Y, F2;
+  FL_RC(G.alloc(c.bytes, c.st));
+  FL_RC(old.alloc(c.old_bytes * n, c.st));
+  FL_RC(Y.alloc(c.bytes / 4, c.st));
+  FL_RC(F2.alloc(c.bytes, c.st));
+  auto old_of = [&](int i) { return (Cx<double>*)((char*)old.p + c.old_bytes * i); };
+  FL_CUDA(cudaMemcpyAsync(G.p, qgb::field_data(gf0), c.bytes, cudaMemcpyDeviceToDevice, c.st));
   for (int i = 0; i < n; ++i) {
-    FL_CUDA(cudaMemcpyAsync(G[i + 1].p, G[i].p, c.bytes, cudaMemcpyDeviceToDevice, c.st));
-    FL_RC(flow_step_dev(c, G[i + 1].p, C.p, steps[i], false));
-  }
-  if (pre) {
-    FL_RC(qgb_field_copy(gm_force, pre));
-  } else {
-    // the force of the action on the flowed field (set_gm_force, hmc.cpp:466-490)
-    qgb_field* gfl = nullptr;
-    FL_RC(qgb_field_create(&gfl, ts, 4, QGB_KIND_COLOR_MATRIX, QGB_F64));
-    FL_CUDA(cudaMemcpyAsync(qgb::field_data(gfl), G[n].p, c.bytes, cudaMemcpyDeviceToDevice, c.st));
-    int rc = qgb_set_gm_force(gm_force, gfl, beta, c1);
-    qgb_field_destroy(gfl);
-    FL_RC(rc);
+    FlowArgs a = flow_args(c, G.p, steps[i]);
+    a.old = old_of(i);
+    FL_RC(launch_flow_step<FLOW_FORWARD>(c, a, steps[i].flow_size));
   }
   void* F = qgb::field_data(gm_force);
+  if (pre) FL_RC(qgb_field_copy(gm_force, pre));
+  else FL_RC(qgb::force_on(c.g, G.p, F, beta, c1));  // the action's force on the flowed field (hmc.cpp:466-490)
   // back through the steps (set_gm_force_propagated_det_from_flow, flowed-hmc.cpp:1456-1477)
+  void *in = F, *out = F2.p;
   for (int i = n - 1; i >= 0; --i) {
-    const qgb_flow_step& f = steps[i];
-    k_flow_staple<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)G[i].p, (Cx<double>*)C.p, f.mask, f.mu,
-                                              f.flow_size);
+    FlowArgs a = flow_args(c, G.p, steps[i]);
+    a.old = old_of(i);
+    a.Fin = (const Cx<double>*)in;
+    a.Fout = (Cx<double>*)out;
+    a.Y = (Cx<double>*)Y.p;
+    if (with_det) FL_RC(launch_flow_step<FLOW_PULL_DET>(c, a, steps[i].flow_size));
+    else FL_RC(launch_flow_step<FLOW_PULL>(c, a, steps[i].flow_size));
+    const dim3 grid((unsigned)((c.V + 127) / 128), 4);
+    if (steps[i].flow_size == 1)
+      k_flow_force_step<1><<<grid, 128, 0, c.st>>>(c.g, a.U, a.Y, a.Fin, a.Fout, a.mask, a.mu);
+    else
+      k_flow_force_step<2><<<grid, 128, 0, c.st>>>(c.g, a.U, a.Y, a.Fin, a.Fout, a.mask, a.mu);
     FL_CUDA(cudaGetLastError());
-    k_flow_link_tables<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)G[i].p, (const Cx<double>*)C.p, f.mask,
-                                                   f.mu, f.flow_size, f.epsilon, nullptr, (double*)T.p);
-    FL_CUDA(cudaGetLastError());
-    k_flow_force_step<<<c.blocks, 128, 0, c.st>>>(c.g, (const Cx<double>*)G[i].p, (const Cx<double>*)C.p,
-                                                  (const double*)T.p, (const Cx<double>*)F, (Cx<double>*)F2.p, f.mask,
-                                                  f.mu, f.flow_size, f.epsilon, with_det ? 1 : 0);
-    FL_CUDA(cudaGetLastError());
-    FL_CUDA(cudaMemcpyAsync(F, F2.p, c.bytes, cudaMemcpyDeviceToDevice, c.st));
+    std::swap(in, out);
   }
-  FL_CUDA(cudaStreamSynchronize(c.st));
+  if (in != F) FL_CUDA(cudaMemcpyAsync(F, in, c.bytes, cudaMemcpyDeviceToDevice, c.st));
   return QGB_OK;
 }
 }  // namespace
