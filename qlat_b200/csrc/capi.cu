@@ -19,6 +19,7 @@
 
 #include "../../include/qlat_b200.h"
 #include "kernels.h"
+#include "work_pool.h"
 
 using qgb::ForceArgs;
 using qgb::Geo;
@@ -341,7 +342,7 @@ int clover_slot(const qgb_field* gf, qgb_field* ef, qgb_field* qf, int slot)
 {
   QGB_RC(no_domain(gf, "clover sums"));
   const Geo g = geo_of(gf);
-  const int nb = qgb::reduce_blocks(g);
+  const int nb = qgb::clover_blocks(g);
   QGB_RC(ensure_partials((size_t)nb * 2));
   Prof p("clover", 2);
   if (gf->prec == QGB_F64)
@@ -360,14 +361,16 @@ int topology_5li_slot(const qgb_field* gf, qgb_field* terms, qgb_field* total, i
 {
   QGB_RC(no_domain(gf, "topology_charge_5"));
   const Geo g = geo_of(gf);
-  const int nb = qgb::reduce_blocks(g);
+  const int nb = qgb::clover_blocks(g);
   QGB_RC(ensure_partials((size_t)nb * 5));
-  Prof p("topology_5li");
+  qgb::WorkBuf lines;
+  QGB_TRY_CUDA(lines.alloc(qgb::lines_bytes(g, gf->prec == QGB_F64 ? 8 : 4), g_ctx.stream));
+  Prof p("topology_5li", 3);
   if (gf->prec == QGB_F64)
-    QGB_TRY_CUDA(qgb::launch_topology_5li<double>(g, gf->d, terms ? terms->d : nullptr, total ? total->d : nullptr,
+    QGB_TRY_CUDA(qgb::launch_topology_5li<double>(g, gf->d, lines.p, terms ? terms->d : nullptr, total ? total->d : nullptr,
                                                   g_ctx.partials, g_ctx.stream));
   else
-    QGB_TRY_CUDA(qgb::launch_topology_5li<float>(g, gf->d, terms ? terms->d : nullptr, total ? total->d : nullptr,
+    QGB_TRY_CUDA(qgb::launch_topology_5li<float>(g, gf->d, lines.p, terms ? terms->d : nullptr, total ? total->d : nullptr,
                                                  g_ctx.partials, g_ctx.stream));
   QGB_TRY_CUDA(qgb::launch_finalize(g_ctx.partials, 5, nb, g_ctx.results, slot, g_ctx.stream));
   return QGB_OK;
@@ -841,6 +844,32 @@ int force_on(const Geo& g, const void* U, void* out, double beta, double c1)
 {
   QGB_CTX();
   return force<double>(g, FORCE_SET, fargs(U, out, beta, c1, 0.0));
+}
+cudaError_t work_pool(cudaMemPool_t* out)
+{
+  static std::mutex mu;
+  static cudaMemPool_t pools[64] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= 64) return cudaErrorInvalidDevice;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!pools[dev]) {
+    cudaMemPoolProps props;
+    memset(&props, 0, sizeof(props));
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    e = cudaMemPoolCreate(&p, &props);
+    if (e != cudaSuccess) return e;
+    uint64_t keep = (uint64_t)1 << 30;
+    e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (e != cudaSuccess) return e;
+    pools[dev] = p;
+  }
+  *out = pools[dev];
+  return cudaSuccess;
 }
 // Lets the allocation-free entry point (noalloc.cu) report through qgb_last_error.
 void set_last_error(const std::string& msg) { g_err = msg; }

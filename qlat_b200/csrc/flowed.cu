@@ -25,7 +25,6 @@
 #include <stdint.h>
 #include <string.h>
 
-#include <mutex>
 #include <string>
 #include <utility>
 #include <vector>
@@ -33,6 +32,7 @@
 #include "../../include/qlat_b200.h"
 #include "gauge_common.cuh"
 #include "kernels.h"
+#include "work_pool.h"
 
 namespace qgb
 {
@@ -623,53 +623,6 @@ int check_steps(const Geo& g, const qgb_flow_step* steps, int n)
   return QGB_OK;
 }
 
-// Work buffers of one call, in stream order.  The pool keeps at most 1 GiB from call to call (beyond that the
-// memory goes back to the device when the stream is next synchronised), and every call owns its buffers, so
-// calls of several threads do not share them.
-int work_pool(cudaMemPool_t* out)
-{
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
-  int dev = 0;
-  FL_CUDA(cudaGetDevice(&dev));
-  if (dev >= 64) return ffail(QGB_ERR_CUDA, "flowed: device number out of range");
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
-    cudaMemPoolProps props;
-    memset(&props, 0, sizeof(props));
-    props.allocType = cudaMemAllocationTypePinned;
-    props.location.type = cudaMemLocationTypeDevice;
-    props.location.id = dev;
-    cudaMemPool_t p = nullptr;
-    FL_CUDA(cudaMemPoolCreate(&p, &props));
-    uint64_t keep = (uint64_t)1 << 30;
-    FL_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep));
-    pools[dev] = p;
-  }
-  *out = pools[dev];
-  return QGB_OK;
-}
-
-struct DevBuf {
-  void* p = nullptr;
-  cudaStream_t st = nullptr;
-  DevBuf() = default;
-  DevBuf(const DevBuf&) = delete;
-  DevBuf& operator=(const DevBuf&) = delete;
-  ~DevBuf()
-  {
-    if (p) cudaFreeAsync(p, st);
-  }
-  int alloc(size_t b, cudaStream_t stream)
-  {
-    cudaMemPool_t pool = nullptr;
-    FL_RC(work_pool(&pool));
-    st = stream;
-    FL_CUDA(cudaMallocFromPoolAsync(&p, b > 0 ? b : 1, pool, stream));
-    return QGB_OK;
-  }
-};
-
 int setup(FlowCtx& c, const qgb_field* gf, int32_t n, const qgb_flow_step* steps)
 {
   int32_t ts[4], mult = 0, kind = 0, prec = 0;
@@ -810,9 +763,9 @@ int qgb_gf_flow_and_ln_det_node(qgb_field* gf, const qgb_field* gf0, const qgb_f
   if (!ln_det) return ffail(QGB_ERR_INVALID_ARG, "qgb_gf_flow_and_ln_det_node: null output");
   FL_RC(check_output(gf));
   FL_RC(qgb_field_copy(gf, gf0));
-  DevBuf L, S;
-  FL_RC(L.alloc((size_t)c.links * sizeof(double) * (n > 0 ? n : 1), c.st));
-  FL_RC(S.alloc((size_t)(n > 0 ? n : 1) * sizeof(double), c.st));
+  WorkBuf L, S;
+  FL_CUDA(L.alloc((size_t)c.links * sizeof(double) * (n > 0 ? n : 1), c.st));
+  FL_CUDA(S.alloc((size_t)(n > 0 ? n : 1) * sizeof(double), c.st));
   void* U = qgb::field_data(gf);
   for (int i = 0; i < n; ++i) {
     FlowArgs a = flow_args(c, U, steps[i]);
@@ -869,11 +822,11 @@ int flowed_force(qgb_field* gm_force, const qgb_field* gf0, const qgb_field* pre
                                    "gauge field's lattice");
   // one work field: the flow runs in it and keeps the links that each step replaces (an eighth of the field), and
   // the way back puts them in place again
-  DevBuf G, old, Y, F2;
-  FL_RC(G.alloc(c.bytes, c.st));
-  FL_RC(old.alloc(c.old_bytes * n, c.st));
-  FL_RC(Y.alloc(c.bytes / 4, c.st));
-  FL_RC(F2.alloc(c.bytes, c.st));
+  WorkBuf G, old, Y, F2;
+  FL_CUDA(G.alloc(c.bytes, c.st));
+  FL_CUDA(old.alloc(c.old_bytes * n, c.st));
+  FL_CUDA(Y.alloc(c.bytes / 4, c.st));
+  FL_CUDA(F2.alloc(c.bytes, c.st));
   auto old_of = [&](int i) { return (Cx<double>*)((char*)old.p + c.old_bytes * i); };
   FL_CUDA(cudaMemcpyAsync(G.p, qgb::field_data(gf0), c.bytes, cudaMemcpyDeviceToDevice, c.st));
   for (int i = 0; i < n; ++i) {

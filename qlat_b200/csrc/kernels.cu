@@ -437,234 +437,6 @@ cudaError_t launch_action(const Geo& g, const void* U, int rect, double* partial
   return cudaGetLastError();
 }
 
-// Clover leaf sum C_mu_nu(x) (the 4 leaves of qcd-acc.h:135-150, without the 1/4).
-template <typename R>
-__device__ __forceinline__ M3<R> clover_sum(const CField<R>& U, const Geo& g, const Coord& x, long s, int mu, int nu)
-{
-  // leaf 1: (mu, nu, -mu, -nu) = U_mu(x) U_nu(x+mu) [U_nu(x) U_mu(x+nu)]^+
-  M3<R> C = mul_adj(mul(U.ld(s, mu), U.ld(site_rt(g, x, mu, 1, nu, 0), nu)),
-                    mul(U.ld(s, nu), U.ld(site_rt(g, x, mu, 0, nu, 1), mu)));
-  // leaf 2: (-mu, -nu, mu, nu) = [U_nu(x-mu-nu) U_mu(x-mu)]^+ U_mu(x-mu-nu) U_nu(x-nu)
-  {
-    const M3<R> a = mul(U.ld(site_rt(g, x, mu, -1, nu, -1), nu), U.ld(site_rt(g, x, mu, -1, nu, 0), mu));
-    const M3<R> b = mul(U.ld(site_rt(g, x, mu, -1, nu, -1), mu), U.ld(site_rt(g, x, mu, 0, nu, -1), nu));
-    C = add_adj_mul(C, a, b);
-  }
-  // leaf 3: (nu, -mu, -nu, mu) = U_nu(x) U_mu(x-mu+nu)^+ U_nu(x-mu)^+ U_mu(x-mu)
-  {
-    const M3<R> a = mul_adj(U.ld(s, nu), U.ld(site_rt(g, x, mu, -1, nu, 1), mu));
-    const M3<R> b = adj_mul(U.ld(site_rt(g, x, mu, -1, nu, 0), nu), U.ld(site_rt(g, x, mu, -1, nu, 0), mu));
-    C = add_mul(C, a, b);
-  }
-  // leaf 4: (-nu, mu, nu, -mu) = U_nu(x-nu)^+ U_mu(x-nu) U_nu(x-nu+mu) U_mu(x)^+
-  {
-    const M3<R> a = adj_mul(U.ld(site_rt(g, x, mu, 0, nu, -1), nu), U.ld(site_rt(g, x, mu, 0, nu, -1), mu));
-    const M3<R> b = mul_adj(U.ld(site_rt(g, x, mu, 1, nu, -1), nu), U.ld(s, mu));
-    C = add_mul(C, a, b);
-  }
-  return C;
-}
-
-// (C - C^+)/8 = the anti-Hermitian part of the leaf average C/4.
-template <typename R>
-__device__ __forceinline__ M3<R> leaf_antiherm(const M3<R>& C)
-{
-  M3<R> ah;
-#pragma unroll
-  for (int r = 0; r < 3; ++r)
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      ah.e[3 * r + c] = cx<R>(R(0.125) * (C.e[3 * r + c].re - C.e[3 * c + r].re),
-                             R(0.125) * (C.e[3 * r + c].im + C.e[3 * c + r].im));
-  return ah;
-}
-
-// -tr(G^2) with G = TA(C/4) = Fa - i Im(tr Fa)/3 (matrix-hmc.h:202-213)
-template <typename R>
-__device__ __forceinline__ double energy_of(const M3<R>& Fa)
-{
-  M3<R> G = Fa;
-  const R t = (G.e[0].im + G.e[4].im + G.e[8].im) / R(3);
-  G.e[0].im -= t;
-  G.e[4].im -= t;
-  G.e[8].im -= t;
-  return -(double)re_tr_mul(G, G);
-}
-
-// Energy density E(x) = sum_{mu<nu} -tr(G_mu_nu^2), G = TA(C/4)
-// (wilson-flow.cpp:99-129) and the clover topological charge density
-// -1/(4 pi^2) [-tr(F02 F13) + tr(F03 F12) + tr(F23 F01)], F = (C/4 - C^+/4)/2
-// (qcd.cpp:64-79), sharing the leaves; planes are visited in the pairs the
-// charge needs so that only two plane matrices are live at a time.
-template <typename R>
-__global__ void __launch_bounds__(RED_BS) k_clover(Geo g, const Cx<R>* Up, R* ef, R* qf, double* partials)
-{
-  const long s = site_of_work(g, (long)blockIdx.x * blockDim.x + threadIdx.x, RED_BS);
-  double v[2] = {0.0, 0.0};
-  if (s < g.V && in_reduce(g, s)) {
-    const CField<R> U{Up, g.V};
-    const Coord x = coord_of(g, s);
-    double e = 0.0, q = 0.0;
-    // plane pairs (02,13) -, (03,12) +, (23,01) +
-#pragma unroll 1
-    for (int p = 0; p < 3; ++p) {
-      const int m1 = p == 2 ? 2 : 0, n1 = p == 0 ? 2 : (p == 1 ? 3 : 3);
-      const int m2 = p == 2 ? 0 : 1, n2 = p == 0 ? 3 : (p == 1 ? 2 : 1);
-      const M3<R> Fa = leaf_antiherm(clover_sum<R>(U, g, x, s, m1, n1));
-      const M3<R> Fb = leaf_antiherm(clover_sum<R>(U, g, x, s, m2, n2));
-      e += energy_of(Fa) + energy_of(Fb);
-      const double t = (double)re_tr_mul(Fa, Fb);
-      q += p == 0 ? -t : t;
-    }
-    q *= -1.0 / (4.0 * 3.141592653589793 * 3.141592653589793);
-    v[0] = e;
-    v[1] = q;
-    if (ef) ef[s] = (R)e;
-    if (qf) qf[s] = (R)q;
-  }
-  block_reduce_store<2>(v, partials);
-}
-
-template <typename R>
-cudaError_t launch_clover(const Geo& g, const void* U, void* e_field, void* q_field, double* partials,
-                          cudaStream_t st)
-{
-  // the grid covers every site of the field: a domain's owned-box traversal does not apply here
-  if (has_box(g)) return cudaErrorInvalidValue;
-  Geo gk = g;  // z slabs on large lattices (the leaves reach one slice either way)
-  set_slab_order(gk, RED_BS, (int)(18 * sizeof(R)));
-  k_clover<R><<<reduce_blocks(g), RED_BS, 0, st>>>(gk, (const Cx<R>*)U, (R*)e_field, (R*)q_field, partials);
-  return cudaGetLastError();
-}
-
-// ------------------------------------------------------------------------
-// 5-loop improved topological charge (qcd.cpp:425-489, hep-lat/9701012)
-
-// Site index of x + the offsets (o0, o1, o2, o3), periodic.
-__device__ __forceinline__ long site_of4(const Geo& g, int y0, int y1, int y2, int y3)
-{
-  return (long)y0 + (long)g.d[0] * ((long)y1 + (long)g.d[1] * ((long)y2 + (long)g.d[2] * (long)y3));
-}
-
-// Sum of the four m x n leaves at x in the (mu, nu) plane (qcd.cpp:11-31,
-// without its 1/4): each a Wilson line of qcd-acc.h:23-41 walked link by link
-// -- forward steps multiply by U_dir(y), backward steps by U_dir(y - dir)^+.
-template <typename R>
-__device__ M3<R> leaf_sum_mn(const CField<R>& U, const Geo& g, const Coord& x, int mu, int m, int nu, int n)
-{
-  M3<R> acc = m3_zero<R>();
-#pragma unroll 1
-  for (int l = 0; l < 4; ++l) {
-    // leaves (mu m, nu n, -mu m, -nu n), (-mu m, -nu n, mu m, nu n),
-    //        (nu n, -mu m, -nu n, mu m), (-nu n, mu m, nu n, -mu m)
-    const int first = l < 2 ? mu : nu, second = l < 2 ? nu : mu;
-    const int cf = l < 2 ? m : n, cs = l < 2 ? n : m;
-    const int sf = (l == 0 || l == 2) ? 1 : -1;  // sign of the first leg
-    const int ss = (l == 0 || l == 3) ? 1 : -1;  // sign of the second leg
-    int y0 = x.c[0], y1 = x.c[1], y2 = x.c[2], y3 = x.c[3];
-    M3<R> w = m3_unit<R>();
-    bool first_link = true;
-#pragma unroll 1
-    for (int leg = 0; leg < 4; ++leg) {
-      const int dir = (leg & 1) ? second : first;
-      const int cnt = (leg & 1) ? cs : cf;
-      const int sgn = ((leg & 1) ? ss : sf) * (leg < 2 ? 1 : -1);
-#pragma unroll 1
-      for (int r = 0; r < cnt; ++r) {
-        if (sgn < 0) {
-          y0 = dir == 0 ? wrap(y0 - 1, g.d[0]) : y0;
-          y1 = dir == 1 ? wrap(y1 - 1, g.d[1]) : y1;
-          y2 = dir == 2 ? wrap(y2 - 1, g.d[2]) : y2;
-          y3 = dir == 3 ? wrap(y3 - 1, g.d[3]) : y3;
-        }
-        const M3<R> u = U.ld(site_of4(g, y0, y1, y2, y3), dir);
-        if (first_link) w = sgn > 0 ? u : adj(u);  // 1 * u is u exactly
-        else w = sgn > 0 ? mul(w, u) : mul_adj(w, u);
-        first_link = false;
-        if (sgn > 0) {
-          y0 = dir == 0 ? wrap(y0 + 1, g.d[0]) : y0;
-          y1 = dir == 1 ? wrap(y1 + 1, g.d[1]) : y1;
-          y2 = dir == 2 ? wrap(y2 + 1, g.d[2]) : y2;
-          y3 = dir == 3 ? wrap(y3 + 1, g.d[3]) : y3;
-        }
-      }
-    }
-    add_to(acc, w);
-  }
-  return acc;
-}
-
-// F = (C - C^+)/2 of the (averaged) m x n leaf C of plane p (qcd.cpp:536-568)
-template <typename R>
-__device__ M3<R> leaf_f_mn(const CField<R>& U, const Geo& g, const Coord& x, int p, int m, int n)
-{
-  const int mu = p < 3 ? 0 : (p < 5 ? 1 : 2);
-  const int nu = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
-  M3<R> c = scale(R(0.25), leaf_sum_mn(U, g, x, mu, m, nu, n));
-  if (m != n) {
-    add_to(c, scale(R(0.25), leaf_sum_mn(U, g, x, mu, n, nu, m)));
-    c = scale(R(0.5), c);
-  }
-  M3<R> f;
-#pragma unroll
-  for (int i = 0; i < 3; ++i)
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      f.e[3 * i + j] = cx<R>(R(0.5) * (c.e[3 * i + j].re - c.e[3 * j + i].re),
-                             R(0.5) * (c.e[3 * i + j].im + c.e[3 * j + i].im));
-  return f;
-}
-
-// Per site the five terms c_k / (m n)^2 * q_{m x n} (terms field, multiplicity
-// 5, optional), their per-site sum (total field, optional), and the block
-// partial sums of the five terms.
-template <typename R>
-__global__ void __launch_bounds__(RED_BS) k_topology_5li(Geo g, const Cx<R>* Up, R* terms, R* total, double* partials)
-{
-  const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (s < g.V) {
-    const CField<R> U{Up, g.V};
-    const Coord x = coord_of(g, s);
-    const double c5 = 1.0 / 20.0;
-    const double coef[5] = {(19.0 - 55.0 * c5) / 9.0, (1.0 - 64.0 * c5) / 9.0 / 16.0,
-                            (-64.0 + 640.0 * c5) / 45.0 / 4.0, (1.0 / 5.0 - 2.0 * c5) / 9.0, c5 / 81.0};
-    const double fac = -1.0 / (4.0 * 3.141592653589793 * 3.141592653589793);
-    double tot = 0.0;
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const int m = k == 1 ? 2 : (k == 4 ? 3 : 1);
-      const int n = k == 0 ? 1 : (k == 1 ? 2 : (k == 2 ? 2 : 3));
-      double q = 0.0;
-      // qcd.cpp:64-79: -tr(F02 F13) + tr(F03 F12) + tr(F23 F01)
-#pragma unroll 1
-      for (int pr = 0; pr < 3; ++pr) {
-        const int pa = pr == 0 ? 1 : (pr == 1 ? 2 : 5), pb = pr == 0 ? 4 : (pr == 1 ? 3 : 0);
-        const M3<R> fa = leaf_f_mn(U, g, x, pa, m, n);
-        const M3<R> fb = leaf_f_mn(U, g, x, pb, m, n);
-        const double t = (double)re_tr_mul(fa, fb);
-        q += pr == 0 ? -t : t;
-      }
-      v[k] = coef[k] * (fac * q);
-      tot += v[k];
-    }
-    if (terms) {
-#pragma unroll
-      for (int k = 0; k < 5; ++k) terms[lay_index<1>(g.V, k, 0, s)] = (R)v[k];
-    }
-    if (total) total[s] = (R)tot;
-  }
-  block_reduce_store<5>(v, partials);
-}
-
-template <typename R>
-cudaError_t launch_topology_5li(const Geo& g, const void* U, void* terms, void* total, double* partials,
-                                cudaStream_t st)
-{
-  k_topology_5li<R><<<reduce_blocks(g), RED_BS, 0, st>>>(g, (const Cx<R>*)U, (R*)terms, (R*)total, partials);
-  return cudaGetLastError();
-}
-
 template <typename R>
 __global__ void __launch_bounds__(RED_BS) k_qnorm(long n, const R* x, double* partials)
 {
@@ -683,30 +455,30 @@ cudaError_t launch_qnorm(long n_reals, const void* x, double* partials, int bloc
   return cudaGetLastError();
 }
 
-__global__ void __launch_bounds__(1024) k_finalize(const double* partials, int nv, int blocks, double* results,
-                                                   int slot)
+// One block per value: its partial sums in a fixed order (loads in groups of 8, so that a block's latency is
+// paid once per group).
+__global__ void __launch_bounds__(1024) k_finalize(const double* partials, int blocks, double* results, int slot)
 {
   __shared__ double sm[32];
-  for (int k = 0; k < nv; ++k) {
-    double t = 0.0;
-    for (int i = threadIdx.x; i < blocks; i += blockDim.x) t += partials[(long)k * blocks + i];
+  const int k = blockIdx.x;
+  double t = 0.0;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < blocks; i += 1024) t += partials[(long)k * blocks + i];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double r = 0.0;
-      for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r += sm[i];
-      results[slot + k] = r;
-    }
-    __syncthreads();
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double r = 0.0;
+    for (int i = 0; i < 32; ++i) r += sm[i];
+    results[slot + k] = r;
   }
 }
 
 cudaError_t launch_finalize(const double* partials, int n_values, int blocks, double* results, int slot,
                             cudaStream_t st)
 {
-  k_finalize<<<1, 1024, 0, st>>>(partials, n_values, blocks, results, slot);
+  k_finalize<<<n_values, 1024, 0, st>>>(partials, blocks, results, slot);
   return cudaGetLastError();
 }
 
@@ -1172,8 +944,6 @@ cudaError_t launch_convert(long n, const void* in, void* out, cudaStream_t st)
   template cudaError_t launch_evolve<R>(const Geo&, void*, const void*, double, int, int, cudaStream_t);    \
   template cudaError_t launch_gm_hamilton<R>(const Geo&, const void*, double*, cudaStream_t);              \
   template cudaError_t launch_action<R>(const Geo&, const void*, int, double*, cudaStream_t, void*);       \
-  template cudaError_t launch_clover<R>(const Geo&, const void*, void*, void*, double*, cudaStream_t);     \
-  template cudaError_t launch_topology_5li<R>(const Geo&, const void*, void*, void*, double*, cudaStream_t); \
   template cudaError_t launch_qnorm<R>(long, const void*, double*, int, cudaStream_t);                    \
   template cudaError_t launch_rand_momentum<R>(const Geo&, void*, const uint32_t*, double, int*, cudaStream_t); \
   template cudaError_t launch_hot_start<R>(const Geo&, void*, const uint32_t*, double, int, int*, cudaStream_t); \

@@ -173,14 +173,18 @@ cudaError_t launch_unitarize_to_f64(const Geo& g, const void* P, void* Q, cudaSt
 template <typename R>
 cudaError_t launch_action(const Geo& g, const void* U, int rect, double* partials, cudaStream_t st,
                           void* copy_f32 = nullptr);
+// Clover and improved-charge sums (clover.cu): clover_blocks(g) partial sums per value.
+int clover_blocks(const Geo& g);
 // values: 0 = energy density sum, 1 = clover topological charge sum; optional fields
 template <typename R>
 cudaError_t launch_clover(const Geo& g, const void* U, void* e_field, void* q_field, double* partials,
                           cudaStream_t st);
 // values 0..4: the five terms of the 5-loop improved charge (qcd.cpp:425-489);
-// optional fields: terms (real, multiplicity 5) and their per-site sum (multiplicity 1)
+// optional fields: terms (real, multiplicity 5) and their per-site sum (multiplicity 1);
+// lines: work buffer of lines_bytes(g, sizeof(R)) bytes
+size_t lines_bytes(const Geo& g, size_t real);
 template <typename R>
-cudaError_t launch_topology_5li(const Geo& g, const void* U, void* terms, void* total, double* partials,
+cudaError_t launch_topology_5li(const Geo& g, const void* U, void* lines, void* terms, void* total, double* partials,
                                 cudaStream_t st);
 template <typename R>
 cudaError_t launch_qnorm(long n_reals, const void* x, double* partials, int blocks, cudaStream_t st);
