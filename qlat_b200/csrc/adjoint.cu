@@ -146,13 +146,197 @@ struct SmemAcc {
   }
 };
 
+// ---- the plaquette force's pull-back ------------------------------------------
+//
+// With V = H W, W = M K^+ the staple of direction +nu (H = U_nu(x), M = U_mu(x+nu), K = U_nu(x+mu)) and
+// W = M K, V = H^+ W that of -nu (H = U_nu(x-nu), M = U_mu(x-nu), K = U_nu(x-nu+mu)), the tangents Y of the
+// links give
+//   +nu: dV = Y_H V + H (Y_M W - W Y_K)
+//   -nu: dV = H^+ ((Y_M - Y_H) W + M (Y_K K))
+// 6 products per direction, 3 of them with an anti-Hermitian factor, where dual matrices
+// (k_force_vjp_rect) take 9 full ones: the kernel is bound by the FP64 pipe, 3900 multiply-adds per link
+// instead of 6600.  S and dS accumulate in shared memory, which leaves the registers to the products
+// (3 blocks of 128 threads per SM).  The four directions of a site block run back to back and meet in L2.
+// 16^4 FP64: 0.188 -> 0.112 ms a launch.
+
+// An su(3) matrix by its diagonal and upper triangle; the products use that the diagonal is imaginary.
+template <typename R>
+struct AntiH {
+  R d[3];
+  Cx<R> o[3];  // (0,1), (0,2), (1,2)
+};
+
+template <typename R>
+__device__ __forceinline__ Cx<R> ah_entry(const AntiH<R>& a, int i, int j)  // i != j
+{
+  const Cx<R> v = a.o[i + j - 1];
+  return i < j ? v : cx<R>(-v.re, v.im);
+}
+
+template <typename R, typename I>
+__device__ __forceinline__ AntiH<R> ld_ah(const CompLd<R, I>& Y, I site)
+{
+  const Cx<R>* q = Y.p + ((site >> 5) * 288 + (site & 31));
+  AntiH<R> a;
+  a.d[0] = ldg_cx(q).im;
+  a.o[0] = ldg_cx(q + 32);
+  a.o[1] = ldg_cx(q + 64);
+  a.d[1] = ldg_cx(q + 32 * 4).im;
+  a.o[2] = ldg_cx(q + 32 * 5);
+  a.d[2] = ldg_cx(q + 32 * 8).im;
+  return a;
+}
+
+// s + a b
+template <typename R>
+__device__ __forceinline__ M3<R> add_ah_mul(const M3<R>& s, const AntiH<R>& a, const M3<R>& b)
+{
+  M3<R> c;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      R re = fma(-a.d[i], b.e[3 * i + j].im, s.e[3 * i + j].re);
+      R im = fma(a.d[i], b.e[3 * i + j].re, s.e[3 * i + j].im);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k == i) continue;
+        const Cx<R> v = ah_entry(a, i, k);
+        re = fma(v.re, b.e[3 * k + j].re, fma(-v.im, b.e[3 * k + j].im, re));
+        im = fma(v.re, b.e[3 * k + j].im, fma(v.im, b.e[3 * k + j].re, im));
+      }
+      c.e[3 * i + j] = cx<R>(re, im);
+    }
+  return c;
+}
+
+// -(b a)
+template <typename R>
+__device__ __forceinline__ M3<R> minus_mul_ah(const M3<R>& b, const AntiH<R>& a)
+{
+  M3<R> c;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      R re = a.d[j] * b.e[3 * i + j].im;
+      R im = -a.d[j] * b.e[3 * i + j].re;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        if (k == j) continue;
+        const Cx<R> v = ah_entry(a, k, j);
+        re = fma(-v.re, b.e[3 * i + k].re, fma(v.im, b.e[3 * i + k].im, re));
+        im = fma(-v.re, b.e[3 * i + k].im, fma(-v.im, b.e[3 * i + k].re, im));
+      }
+      c.e[3 * i + j] = cx<R>(re, im);
+    }
+  return c;
+}
+
+template <typename R>
+__device__ __forceinline__ AntiH<R> ah_sub(AntiH<R> a, const AntiH<R>& b)
+{
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    a.d[i] -= b.d[i];
+    a.o[i].re -= b.o[i].re;
+    a.o[i].im -= b.o[i].im;
+  }
+  return a;
+}
+
+template <typename R>
+__device__ __forceinline__ M3<R> sm_ld(Cx<R> (*m)[128])
+{
+  M3<R> r;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) r.e[k] = m[k][threadIdx.x];
+  return r;
+}
+
+template <typename R>
+__device__ __forceinline__ void sm_st(Cx<R> (*m)[128], const M3<R>& r)
+{
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m[k][threadIdx.x] = r.e[k];
+}
+
+// lambda_out = lambda_local + a (DF[Y] + [F, Y]), F the plaquette action's force; Y and lambda_local in su(3).
+template <typename R, typename I>
+__global__ void __launch_bounds__(128, sizeof(R) == 8 ? 3 : 4)
+    k_force_vjp_plaq(Geo g, const Cx<R>* Up, const Cx<R>* Yp, const Cx<R>* lam_local, Cx<R>* lam_out, double beta, double a)
+{
+  const long w = (long)(blockIdx.x >> 2) * 128 + threadIdx.x;
+  if (w >= g.V) return;
+  const int mu = blockIdx.x & 3;
+  const I s = (I)w;
+  const I comp = (I)site_blocks(g.V) * 288;
+  const Coord x = coord_of(g, w);
+  const CompLd<R, I> Um{Up + mu * comp}, Ym{Yp + mu * comp};
+  const I smu = site_stride<I>(g, mu);
+  const I dmu = nb_offset<I>(sel4(x.c, mu), 1, sel4(g.d, mu), smu);
+  __shared__ Cx<R> sh_s[9][128], sh_ds[9][128];
+  sm_st(sh_s, m3_zero<R>());
+  sm_st(sh_ds, m3_zero<R>());
+#pragma unroll 1
+  for (int i = 1; i < 4; ++i) {
+    const int nu = (mu + i) & 3;
+    const I snu = site_stride<I>(g, nu);
+    const CompLd<R, I> Un{Up + nu * comp}, Yn{Yp + nu * comp};
+    {
+      const I y = s + nb_offset<I>(sel4(x.c, nu), 1, sel4(g.d, nu), snu);
+      const M3<R> W = mul_adj(Um(y), Un(s + dmu));
+      const M3<R> T = add_ah_mul(minus_mul_ah(W, ld_ah(Yn, s + dmu)), ld_ah(Ym, y), W);
+      const M3<R> H = Un(s);
+      sm_st(sh_ds, add_mul(sm_ld(sh_ds), H, T));
+      const M3<R> V = mul(H, W);
+      sm_st(sh_ds, add_ah_mul(sm_ld(sh_ds), ld_ah(Yn, s), V));
+      M3<R> S = sm_ld(sh_s);
+      add_to(S, V);
+      sm_st(sh_s, S);
+    }
+    {
+      const I y = s + nb_offset<I>(sel4(x.c, nu), -1, sel4(g.d, nu), snu);
+      const M3<R> K = Un(y + dmu), M = Um(y);
+      const M3<R> W = mul(M, K);
+      M3<R> T = mul(M, add_ah_mul(m3_zero<R>(), ld_ah(Yn, y + dmu), K));
+      T = add_ah_mul(T, ah_sub(ld_ah(Ym, y), ld_ah(Yn, y)), W);
+      const M3<R> H = Un(y);
+      sm_st(sh_ds, add_adj_mul(sm_ld(sh_ds), H, T));
+      sm_st(sh_s, add_adj_mul(sm_ld(sh_s), H, W));
+    }
+  }
+  // DF[Y] = c TA(Y (U S^+) + U dS^+), and [F, Y] by structure constants
+  const M3<R> u = Um(s);
+  const AntiH<R> y = ld_ah(Ym, s);
+  const M3<R> P = mul_adj(u, sm_ld(sh_s));
+  const M3<R> D = traceless_antiherm(add_ah_mul(mul_adj(u, sm_ld(sh_ds)), y, P));
+  R f[8], d[8], yb[8], out[8], l[8];
+  su3_coefs(traceless_antiherm(P), f);
+  su3_coefs(D, d);
+  M3<R> ym;
+  ym.e[0].im = y.d[0];
+  ym.e[4].im = y.d[1];
+  ym.e[1] = y.o[0];
+  ym.e[2] = y.o[1];
+  ym.e[5] = y.o[2];
+  su3_coefs(ym, yb);
+  minus_ad(out, yb, f);
+  su3_coefs(CField<R>{lam_local, g.V}.ld(w, mu), l);
+  const R c = R(-beta / 3.0) * R(a);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) out[k] = fma(c, out[k] + d[k], l[k]);
+  WField<R>{lam_out, g.V}.st(w, mu, su3_matrix(out));
+}
+
+// ---- the same with rectangles: every path as a product of dual matrices --------
+
 // lambda_out = lambda_local + a (DF[Y] + [F, Y]) at every link, F the force
 // of GaugeAction(beta, c1) (hmc.cpp:48-75: staples (1 - 8 c1) plaq + c1 rect,
-// the paths of hmc.cpp:27-46), DF[Y] its derivative along Y, every path
-// walked as a product of dual matrices.
-template <typename R, bool RECT>
-__global__ void __launch_bounds__(128) k_force_vjp(Geo g, const Cx<R>* Up, const Cx<R>* Yp, const Cx<R>* lam_local,
-                                                   Cx<R>* lam_out, double beta, double c1, double a)
+// the paths of hmc.cpp:27-46), DF[Y] its derivative along Y.
+template <typename R>
+__global__ void __launch_bounds__(128) k_force_vjp_rect(Geo g, const Cx<R>* Up, const Cx<R>* Yp, const Cx<R>* lam_local,
+                                                        Cx<R>* lam_out, double beta, double c1, double a)
 {
   const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= g.V) return;
@@ -168,23 +352,21 @@ __global__ void __launch_bounds__(128) k_force_vjp(Geo g, const Cx<R>* Up, const
     const DualDir<R> d{U, Y, g, x, mu, (mu + 1 + (k >> 1)) & 3, (k & 1) ? -1 : 1};
     // plaq (nu, mu, -nu) = hop(x) U_mu(x+e) back(x+e+mu)
     acc.add(cp, dmul(dmul(d.hop(0, 0), d.umu(0, 1)), d.back(1, 1)));
-    if (RECT) {
-      // rect1 (nu, nu, mu, -nu, -nu)
-      Dual<R> C = dmul(d.hop(0, 0), d.hop(0, 1));
-      C = dmul(C, d.umu(0, 2));
-      C = dmul(C, d.back(1, 2));
-      acc.add(cr, dmul(C, d.back(1, 1)));
-      // rect2 (nu, mu, mu, -nu, -mu)
-      C = dmul(d.hop(0, 0), d.umu(0, 1));
-      C = dmul(C, d.umu(1, 1));
-      C = dmul(C, d.back(2, 1));
-      acc.add(cr, dmul(C, d.umu(1, 0, true)));
-      // rect3 (-mu, nu, mu, mu, -nu)
-      C = dmul(d.umu(-1, 0, true), d.hop(-1, 0));
-      C = dmul(C, d.umu(-1, 1));
-      C = dmul(C, d.umu(0, 1));
-      acc.add(cr, dmul(C, d.back(1, 1)));
-    }
+    // rect1 (nu, nu, mu, -nu, -nu)
+    Dual<R> C = dmul(d.hop(0, 0), d.hop(0, 1));
+    C = dmul(C, d.umu(0, 2));
+    C = dmul(C, d.back(1, 2));
+    acc.add(cr, dmul(C, d.back(1, 1)));
+    // rect2 (nu, mu, mu, -nu, -mu)
+    C = dmul(d.hop(0, 0), d.umu(0, 1));
+    C = dmul(C, d.umu(1, 1));
+    C = dmul(C, d.back(2, 1));
+    acc.add(cr, dmul(C, d.umu(1, 0, true)));
+    // rect3 (-mu, nu, mu, mu, -nu)
+    C = dmul(d.umu(-1, 0, true), d.hop(-1, 0));
+    C = dmul(C, d.umu(-1, 1));
+    C = dmul(C, d.umu(0, 1));
+    acc.add(cr, dmul(C, d.back(1, 1)));
   }
   const M3<R> S = acc.S(), dS = acc.dS();
   const M3<R> u = U.ld(s, mu);
@@ -197,17 +379,6 @@ __global__ void __launch_bounds__(128) k_force_vjp(Geo g, const Cx<R>* Up, const
   axpy(out, R(a), dF);
   axpy(out, R(a), commutator(F, y));
   WField<R>{lam_out, g.V}.st(s, mu, traceless_antiherm(out));
-}
-
-template <typename R>
-__device__ __forceinline__ M3<R> add_to_copy(M3<R> a, const M3<R>& b)
-{
-#pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    a.e[i].re += b.e[i].re;
-    a.e[i].im += b.e[i].im;
-  }
-  return a;
 }
 
 // dexp_A(B) = sum_{k>=0} ad_A^k B / (k+1)!
@@ -225,6 +396,10 @@ __device__ __forceinline__ M3<R> dexp_apply(const M3<R>& A, const M3<R>& B)
 
 // Link-local part of a stage's pull-back:
 //   mu_out = eps dexp_{-eps Z}(lambda) + carry * mu_carry,   lam_local = e^{-eps Z} lambda e^{eps Z}.
+// lambda counts by its su(3) part (ad_Z of the rest has none); Z and mu_carry are in su(3).  In su(3)
+// coefficients a nested commutator takes 54 multiply-adds instead of 216, so the kernel is bound by
+// memory: five fields, 189 MB at 16^4 in FP64:
+// 0.062 -> 0.027 ms.
 template <typename R>
 __global__ void __launch_bounds__(128) k_flow_adj_local(long V, const Cx<R>* lam, const Cx<R>* Z, const Cx<R>* mu_carry,
                                                         double carry, double eps, Cx<R>* mu_out, Cx<R>* lam_local)
@@ -232,33 +407,45 @@ __global__ void __launch_bounds__(128) k_flow_adj_local(long V, const Cx<R>* lam
   const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= V) return;
   const int mu = blockIdx.y;
-  const M3<R> l = CField<R>{lam, V}.ld(s, mu);
-  const M3<R> A = scale(R(-eps), CField<R>{Z, V}.ld(s, mu));
-  // Both parts from one series of nested commutators c_k = ad_A^k lambda:
+  R l[8], A[8], ad[8], d[8], c[8], t[8];
+  su3_coefs(traceless_antiherm(CField<R>{lam, V}.ld(s, mu)), l);
+  su3_coefs(CField<R>{Z, V}.ld(s, mu), A);
+  // Both parts from one series of nested commutators c_k = ad_A^k lambda, A = -eps Z:
   // dexp_A(lambda) = sum_k c_k / (k+1)! and e^A lambda e^-A = sum_k c_k / k!,
   // cut once |c_k| / k! (Frobenius norms, |ad_A| <= 2 |A|) falls below
   // 2^-60 |lambda| (2^-30 in FP32), under the rounding of either sum.
   R na2 = R(0), nl2 = R(0);
 #pragma unroll
-  for (int i = 0; i < 9; ++i) {
-    na2 = fma(A.e[i].re, A.e[i].re, fma(A.e[i].im, A.e[i].im, na2));
-    nl2 = fma(l.e[i].re, l.e[i].re, fma(l.e[i].im, l.e[i].im, nl2));
+  for (int i = 0; i < 8; ++i) {
+    A[i] *= R(eps);  // minus_ad changes the sign
+    na2 = fma(A[i], A[i], na2);
+    nl2 = fma(l[i], l[i], nl2);
+    c[i] = ad[i] = d[i] = l[i];
   }
-  const R nad = R(2) * sqrt(na2);
+  const R nad = R(2) * sqrt(R(2) * na2);
   const R tol = (sizeof(R) == 4 ? R(9.313225746154785e-10) : R(8.673617379884035e-19)) * sqrt(nl2);
-  M3<R> d = l, ad = l, c = l;
   R bound = sqrt(nl2);  // bound on |c_k| / k!
 #pragma unroll 1
   for (int k = 1; k <= 30 && bound > tol; ++k) {
-    c = scale(R(1) / R(k), commutator(A, c));  // c_k / k!
-    ad = add_to_copy(ad, c);
-    d = add_to_copy(d, scale(R(1) / R(k + 1), c));
-    bound *= nad / R(k);
+    const R inv = R(1) / R(k), inv1 = R(1) / R(k + 1);
+    minus_ad(t, A, c);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      c[i] = t[i] * inv;  // c_k / k!
+      ad[i] += c[i];
+      d[i] = fma(inv1, c[i], d[i]);
+    }
+    bound *= nad * inv;
   }
-  M3<R> m = scale(R(eps), d);
-  if (mu_carry != nullptr && carry != 0.0) axpy(m, R(carry), CField<R>{mu_carry, V}.ld(s, mu));
-  WField<R>{mu_out, V}.st(s, mu, traceless_antiherm(m));
-  WField<R>{lam_local, V}.st(s, mu, traceless_antiherm(ad));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) d[i] *= R(eps);
+  if (mu_carry != nullptr && carry != 0.0) {
+    su3_coefs(CField<R>{mu_carry, V}.ld(s, mu), t);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[i] = fma(R(carry), t[i], d[i]);
+  }
+  WField<R>{mu_out, V}.st(s, mu, su3_matrix(d));
+  WField<R>{lam_local, V}.st(s, mu, su3_matrix(ad));
 }
 
 // out = dexp_{-Omega}(lambda): the gradient with respect to omega of a function
@@ -325,13 +512,11 @@ template <typename R>
 cudaError_t launch_force_vjp(const Geo& g, const void* U, const void* Y, const void* lam_local, void* lam_out,
                              double beta, double c1, double a, cudaStream_t st)
 {
-  dim3 grid((unsigned)((g.V + 127) / 128), 4);
-  if (c1 != 0.0)
-    k_force_vjp<R, true><<<grid, 128, 0, st>>>(g, (const Cx<R>*)U, (const Cx<R>*)Y, (const Cx<R>*)lam_local,
-                                               (Cx<R>*)lam_out, beta, c1, a);
-  else
-    k_force_vjp<R, false><<<grid, 128, 0, st>>>(g, (const Cx<R>*)U, (const Cx<R>*)Y, (const Cx<R>*)lam_local,
-                                                (Cx<R>*)lam_out, beta, 0.0, a);
+  const unsigned nb = (unsigned)((g.V + 127) / 128);
+  const Cx<R>*u = (const Cx<R>*)U, *y = (const Cx<R>*)Y, *l = (const Cx<R>*)lam_local;
+  if (c1 != 0.0) k_force_vjp_rect<R><<<dim3(nb, 4), 128, 0, st>>>(g, u, y, l, (Cx<R>*)lam_out, beta, c1, a);
+  else if (small_offsets(g, 4)) k_force_vjp_plaq<R, int><<<4 * nb, 128, 0, st>>>(g, u, y, l, (Cx<R>*)lam_out, beta, a);
+  else k_force_vjp_plaq<R, long><<<4 * nb, 128, 0, st>>>(g, u, y, l, (Cx<R>*)lam_out, beta, a);
   return cudaGetLastError();
 }
 

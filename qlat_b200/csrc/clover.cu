@@ -99,32 +99,9 @@ __device__ __forceinline__ M3<R> sub_adj_mul(const M3<R>& s, const M3<R>& a, con
   return c;
 }
 
-// Components of a color-matrix field by a site index of type I (int while the field's offsets fit).
-template <typename R, typename I>
-struct Comp {
-  const Cx<R>* p;
-  __device__ __forceinline__ M3<R> operator()(I site) const
-  {
-    const Cx<R>* q = p + ((site >> 5) * 288 + (site & 31));
-    M3<R> r;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) r.e[k] = ldg_cx(q + 32 * k);
-    return r;
-  }
-};
-
-// offset of x + a along one direction (any a, any extent)
-template <typename I>
-__device__ __forceinline__ I delta(int x, int a, int L, I stride)
-{
-  int y = (x + a) % L;
-  if (y < 0) y += L;
-  return (I)(y - x) * stride;
-}
-
 // acc += G at site s; m and n links: am, bn (and amm, bnn) lead m links along a (n along b) forward (backward).
 template <typename R, typename I>
-__device__ __forceinline__ void add_leaves(M3<R>& acc, const Comp<R, I>& A, const Comp<R, I>& B, I s, I am, I amm, I bn,
+__device__ __forceinline__ void add_leaves(M3<R>& acc, const CompLd<R, I>& A, const CompLd<R, I>& B, I s, I am, I amm, I bn,
                                            I bnn)
 {
 #pragma unroll 1
@@ -197,7 +174,6 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3) k_clover(Geo g, co
   const long site = site_of_work(g, valid ? w : g.V - 1, SITES);
   {
     const Coord x = coord_of(g, site);
-    const I st[4] = {1, (I)g.d[0], (I)g.d[0] * g.d[1], (I)g.d[0] * g.d[1] * g.d[2]};
     const I comp = (I)site_blocks(g.V) * 288, s = (I)site;
     double e = 0.0, q = 0.0;
 #pragma unroll 1
@@ -205,10 +181,10 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3) k_clover(Geo g, co
       int a, b;
       plane_of(p, i, a, b);
       const int xa = sel4(x.c, a), xb = sel4(x.c, b), La = sel4(g.d, a), Lb = sel4(g.d, b);
-      const I sa = a == 0 ? st[0] : a == 1 ? st[1] : st[2], sb = b == 1 ? st[1] : b == 2 ? st[2] : st[3];
+      const I sa = site_stride<I>(g, a), sb = site_stride<I>(g, b);
       M3<R> G = m3_zero<R>();
-      add_leaves<R, I>(G, Comp<R, I>{Up + a * comp}, Comp<R, I>{Up + b * comp}, s, delta<I>(xa, 1, La, sa),
-                       delta<I>(xa, -1, La, sa), delta<I>(xb, 1, Lb, sb), delta<I>(xb, -1, Lb, sb));
+      add_leaves<R, I>(G, CompLd<R, I>{Up + a * comp}, CompLd<R, I>{Up + b * comp}, s, nb_offset<I>(xa, 1, La, sa),
+                       nb_offset<I>(xa, -1, La, sa), nb_offset<I>(xb, 1, Lb, sb), nb_offset<I>(xb, -1, Lb, sb));
       const AntiH<R> f = antiherm(R(0.125), G);
       e += (double)energy_of(f);
       if (i == 0) park(sF, f);
@@ -247,15 +223,14 @@ __global__ void __launch_bounds__(128) k_lines(Geo g, const Cx<R>* Up, Cx<R>* li
   if (s >= g.V) return;
   const int a = blockIdx.y;
   const I comp = (I)site_blocks(g.V) * 288;
-  const Comp<R, I> U{Up + a * comp};
+  const CompLd<R, I> U{Up + a * comp};
   const Coord x = coord_of(g, s);
-  const I st[4] = {1, (I)g.d[0], (I)g.d[0] * g.d[1], (I)g.d[0] * g.d[1] * g.d[2]};
   const int xa = sel4(x.c, a), La = sel4(g.d, a);
-  const I sa = a == 0 ? st[0] : a == 1 ? st[1] : a == 2 ? st[2] : st[3];
-  const M3<R> d = mul(U((I)s), U((I)s + delta<I>(xa, 1, La, sa)));
+  const I sa = site_stride<I>(g, a);
+  const M3<R> d = mul(U((I)s), U((I)s + nb_offset<I>(xa, 1, La, sa)));
   const WField<R> L{lines, g.V};
   L.st(s, a, d);
-  L.st(s, 4 + a, mul(d, U((I)s + delta<I>(xa, 2, La, sa))));
+  L.st(s, 4 + a, mul(d, U((I)s + nb_offset<I>(xa, 2, La, sa))));
 }
 
 // The five terms c_k / (m n)^2 q_{m x n} of the improved charge, (m, n) = (1,1), (2,2), (1,2), (1,3), (3,3), the
@@ -275,9 +250,8 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
   const long site = valid ? w : g.V - 1;
   {
     const Coord x = coord_of(g, site);
-    const I st[4] = {1, (I)g.d[0], (I)g.d[0] * g.d[1], (I)g.d[0] * g.d[1] * g.d[2]};
     const I comp = (I)site_blocks(g.V) * 288, s = (I)site;
-    auto line = [&](int a, int m) { return Comp<R, I>{(m == 1 ? Up : lines + (m == 3 ? 4 * comp : (I)0)) + a * comp}; };
+    auto line = [&](int a, int m) { return CompLd<R, I>{(m == 1 ? Up : lines + (m == 3 ? 4 * comp : (I)0)) + a * comp}; };
 #pragma unroll 1
     for (int k = 0; k < 5; ++k) {
       const int m0 = k == 1 ? 2 : (k == 4 ? 3 : 1), n0 = k == 0 ? 1 : (k == 1 || k == 2 ? 2 : 3);
@@ -287,13 +261,13 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
         int a, b;
         plane_of(p, i, a, b);
         const int xa = sel4(x.c, a), xb = sel4(x.c, b), La = sel4(g.d, a), Lb = sel4(g.d, b);
-        const I sa = a == 0 ? st[0] : a == 1 ? st[1] : st[2], sb = b == 1 ? st[1] : b == 2 ? st[2] : st[3];
+        const I sa = site_stride<I>(g, a), sb = site_stride<I>(g, b);
         M3<R> G = m3_zero<R>();
 #pragma unroll 1
         for (int h = 0; h <= (m0 != n0); ++h) {
           const int m = h == 0 ? m0 : n0, n = h == 0 ? n0 : m0;
-          add_leaves<R, I>(G, line(a, m), line(b, n), s, delta<I>(xa, m, La, sa), delta<I>(xa, -m, La, sa),
-                           delta<I>(xb, n, Lb, sb), delta<I>(xb, -n, Lb, sb));
+          add_leaves<R, I>(G, line(a, m), line(b, n), s, nb_offset<I>(xa, m, La, sa), nb_offset<I>(xa, -m, La, sa),
+                           nb_offset<I>(xb, n, Lb, sb), nb_offset<I>(xb, -n, Lb, sb));
         }
         const AntiH<R> f = antiherm(m0 == n0 ? R(0.125) : R(0.0625), G);
         if (i == 0) park(sF, f);
@@ -324,9 +298,6 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
     if (threadIdx.x == 0) partials[(long)k * gridDim.x + blockIdx.x] = r;
   }
 }
-
-// 32-bit offsets reach a field of `mult` color matrices per site
-bool small_offsets(const Geo& g, int mult) { return padded_sites(g.V) * 9 * mult < 2147483647L; }
 
 }  // namespace
 

@@ -46,63 +46,6 @@ namespace
 {
 using namespace qgb;
 
-// ---- su(3) basis (matrix-hmc.h:76-124) and the adjoint representation -------
-
-constexpr double SQRT3 = 1.7320508075688772;
-
-__host__ __device__ inline M3<double> anti_herm_from_basis(const double* b)
-{
-  // make_anti_hermitian_matrix (matrix-hmc.h:76-106)
-  const double s3 = (1.0 / sqrt(3.0)) * b[7];
-  M3<double> m;
-  m.e[0] = cx<double>(0.0, b[2] + s3);
-  m.e[1] = cx<double>(b[1], b[0]);
-  m.e[2] = cx<double>(b[4], b[3]);
-  m.e[3] = cx<double>(-b[1], b[0]);
-  m.e[4] = cx<double>(0.0, -b[2] + s3);
-  m.e[5] = cx<double>(b[6], b[5]);
-  m.e[6] = cx<double>(-b[4], b[3]);
-  m.e[7] = cx<double>(-b[6], b[5]);
-  m.e[8] = cx<double>(0.0, -2.0 * s3);
-  return m;
-}
-
-__host__ __device__ inline void basis_of(const M3<double>& m, double* b)
-{
-  // basis_projection_anti_hermitian_matrix (matrix-hmc.h:108-124)
-  b[0] = m.e[1].im;
-  b[1] = m.e[1].re;
-  b[2] = 0.5 * (m.e[0].im - m.e[4].im);
-  b[3] = m.e[2].im;
-  b[4] = m.e[2].re;
-  b[5] = m.e[5].im;
-  b[6] = m.e[5].re;
-  b[7] = sqrt(3.0) * 0.5 * (m.e[0].im + m.e[4].im);
-}
-
-// r = -ad_x v, the basis coefficients of [v, x] (T_a = i lambda_a, so [T_a, T_b] = -2 f_abc T_c and
-// r_c = 2 sum_ab f_abc x_a v_b): the nine independent structure constants of su(3), 54 multiply-adds
-// on registers instead of an 8 x 8 matrix-vector product.
-__host__ __device__ __forceinline__ void minus_ad(double (&r)[8], const double (&x)[8], const double (&v)[8])
-{
-#pragma unroll
-  for (int c = 0; c < 8; ++c) r[c] = 0.0;
-#define QGB_F(i, j, k, f)                                                              \
-  r[k - 1] = fma(f * x[i - 1], v[j - 1], fma(-(f * x[j - 1]), v[i - 1], r[k - 1]));    \
-  r[i - 1] = fma(f * x[j - 1], v[k - 1], fma(-(f * x[k - 1]), v[j - 1], r[i - 1]));    \
-  r[j - 1] = fma(f * x[k - 1], v[i - 1], fma(-(f * x[i - 1]), v[k - 1], r[j - 1]));
-  QGB_F(1, 2, 3, 2.0)
-  QGB_F(1, 4, 7, 1.0)
-  QGB_F(1, 5, 6, -1.0)
-  QGB_F(2, 4, 6, 1.0)
-  QGB_F(2, 5, 7, 1.0)
-  QGB_F(3, 4, 5, 1.0)
-  QGB_F(3, 6, 7, -1.0)
-  QGB_F(4, 5, 8, SQRT3)
-  QGB_F(6, 7, 8, SQRT3)
-#undef QGB_F
-}
-
 // ---- masks and lattice walks (flowed-hmc.cpp:71-110) ----------------------
 
 // Sites of mask 2 have an even sum of (x_k / size), those of mask 1 an odd one.
@@ -343,7 +286,7 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
     const M3<double> uc = mul_adj(u, c);
     const M3<double> xm = scale(-a.eps, traceless_antiherm(uc));
     double xb[8];
-    basis_of(xm, xb);
+    su3_coefs(xm, xb);
     double nrm = 0.0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) nrm = fma(xb[k], xb[k], nrm);
@@ -369,7 +312,7 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
     double nb[8], mp[8], minv[8], ft[8];
     M3<double> Q = m3_zero<double>();
     if constexpr (DET) {
-      basis_of(traceless_antiherm(mul(anti_herm_from_basis(eb), uc)), nb);
+      su3_coefs(traceless_antiherm(mul(su3_matrix(eb), uc)), nb);
       double* A = sA + w * PAD;
       double* Bm = sB + w * PAD;
       store_col(A, b, jb);
@@ -425,13 +368,13 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
         minus_ad(ft, eb, gb);
 #pragma unroll
         for (int k = 0; k < 8; ++k) ft[k] *= -0.5;
-        Q = scale(0.5, mul(anti_herm_from_basis(eb), anti_herm_from_basis(kb)));
+        Q = scale(0.5, mul(su3_matrix(eb), su3_matrix(kb)));
       }
     }
     if constexpr (PULL) {
       // Z = -W + (E + Q) / 2: W = eps (J(X) F) . T, E = e2dj . T, Q = sum_cb K_cb T_b T_c with K = -eps M'^-1 J(X)
       double fb[8];
-      basis_of(CField<double>{a.Fin, g.V}.ld(s, mu), fb);
+      su3_coefs(CField<double>{a.Fin, g.V}.ld(s, mu), fb);
       double fbb = 0.0;
 #pragma unroll
       for (int k = 0; k < 8; ++k) fbb = k == b ? fb[k] : fbb;
@@ -444,7 +387,7 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
       }
       sum8(z);
       sum8(r);
-      M3<double> Z = anti_herm_from_basis(z);
+      M3<double> Z = su3_matrix(z);
       if constexpr (DET) {
         sum8(Q);
         add_to(Z, Q);
@@ -453,7 +396,7 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
       if (i0 < a.n) {
         if (b == 0) WField<double>{a.Y, g.V}.st(s, 0, mul(Z, u));
         if (b == 1) {
-          M3<double> f = anti_herm_from_basis(r);
+          M3<double> f = su3_matrix(r);
           add_to(f, traceless_antiherm(mul(uc, Z)));
           WField<double>{a.Fout, g.V}.st(s, mu, f);
         }

@@ -213,4 +213,37 @@ __device__ __forceinline__ int sel4(const int (&v)[4], int k)
 
 __device__ __forceinline__ int nb_delta(int xk, int a, int L, int stride) { return (wrap(xk + a, L) - xk) * stride; }
 
+// One component of a color-matrix field (p: its first entry), by a site index of
+// type I: int while the field's offsets fit 31 bits (small_offsets), long else.
+template <typename R, typename I>
+struct CompLd {
+  const Cx<R>* p;
+  __device__ __forceinline__ M3<R> operator()(I site) const
+  {
+    const Cx<R>* q = p + ((site >> 5) * 288 + (site & 31));
+    M3<R> r;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) r.e[k] = ldg_cx(q + 32 * k);
+    return r;
+  }
+};
+
+inline bool small_offsets(const Geo& g, int mult) { return padded_sites(g.V) * 9 * mult < 2147483647L; }
+
+// offset of x + a along one direction, for any a and any extent
+template <typename I>
+__device__ __forceinline__ I nb_offset(int x, int a, int L, I stride)
+{
+  int y = (x + a) % L;
+  if (y < 0) y += L;
+  return (I)(y - x) * stride;
+}
+
+// strides of the site index
+template <typename I>
+__device__ __forceinline__ I site_stride(const Geo& g, int k)
+{
+  return k == 0 ? (I)1 : k == 1 ? (I)g.d[0] : k == 2 ? (I)g.d[0] * g.d[1] : (I)g.d[0] * g.d[1] * g.d[2];
+}
+
 }  // namespace qgb

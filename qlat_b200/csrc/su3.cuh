@@ -747,4 +747,64 @@ QGB_HD M3<R> exp_md(const M3<R>& a)
   return exp_su3(a);
 }
 
+// ---- su(3) matrices as their 8 coefficients (tr T_a T_b = -2 delta_ab) --------
+
+// sum_a b[a] T_a (make_anti_hermitian_matrix, matrix-hmc.h:76-106)
+template <typename R>
+QGB_HD M3<R> su3_matrix(const R (&b)[8])
+{
+  const R s3 = R(0.57735026918962576) * b[7];
+  M3<R> m;
+  m.e[0] = cx<R>(R(0), b[2] + s3);
+  m.e[1] = cx<R>(b[1], b[0]);
+  m.e[2] = cx<R>(b[4], b[3]);
+  m.e[3] = cx<R>(-b[1], b[0]);
+  m.e[4] = cx<R>(R(0), -b[2] + s3);
+  m.e[5] = cx<R>(b[6], b[5]);
+  m.e[6] = cx<R>(-b[4], b[3]);
+  m.e[7] = cx<R>(-b[6], b[5]);
+  m.e[8] = cx<R>(R(0), R(-2) * s3);
+  return m;
+}
+
+// The coefficients of an su(3) matrix, from its diagonal and upper triangle
+// (basis_projection_anti_hermitian_matrix, matrix-hmc.h:108-124).
+template <typename R>
+QGB_HD void su3_coefs(const M3<R>& m, R (&b)[8])
+{
+  b[0] = m.e[1].im;
+  b[1] = m.e[1].re;
+  b[2] = R(0.5) * (m.e[0].im - m.e[4].im);
+  b[3] = m.e[2].im;
+  b[4] = m.e[2].re;
+  b[5] = m.e[5].im;
+  b[6] = m.e[5].re;
+  b[7] = R(0.86602540378443865) * (m.e[0].im + m.e[4].im);
+}
+
+// r = -ad_x v: the coefficients of [v, x].  T_a = i lambda_a, so [T_a, T_b] =
+// -2 f_abc T_c and r_c = 2 sum_ab f_abc x_a v_b, from the nine independent
+// structure constants: 54 multiply-adds, where an 8 x 8 matrix takes 64 and
+// its entries, and a commutator of 3 x 3 matrices 216.
+template <typename R>
+QGB_HD void minus_ad(R (&r)[8], const R (&x)[8], const R (&v)[8])
+{
+#pragma unroll
+  for (int c = 0; c < 8; ++c) r[c] = R(0);
+#define QGB_F(i, j, k, f)                                                                       \
+  r[k - 1] = fma(R(f) * x[i - 1], v[j - 1], fma(-(R(f) * x[j - 1]), v[i - 1], r[k - 1]));       \
+  r[i - 1] = fma(R(f) * x[j - 1], v[k - 1], fma(-(R(f) * x[k - 1]), v[j - 1], r[i - 1]));       \
+  r[j - 1] = fma(R(f) * x[k - 1], v[i - 1], fma(-(R(f) * x[i - 1]), v[k - 1], r[j - 1]));
+  QGB_F(1, 2, 3, 2.0)
+  QGB_F(1, 4, 7, 1.0)
+  QGB_F(1, 5, 6, -1.0)
+  QGB_F(2, 4, 6, 1.0)
+  QGB_F(2, 5, 7, 1.0)
+  QGB_F(3, 4, 5, 1.0)
+  QGB_F(3, 6, 7, -1.0)
+  QGB_F(4, 5, 8, 1.7320508075688772)
+  QGB_F(6, 7, 8, 1.7320508075688772)
+#undef QGB_F
+}
+
 }  // namespace qgb
