@@ -18,6 +18,7 @@
 #include <map>
 #include <string>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "../../include/qlat_b200.h"
@@ -167,13 +168,21 @@ int batch_md(qgb_batch_s* b, void* gf, void* gm, void* tmp, int n_step, double m
       QB_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(b->Vtot) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
                               b->stream));
   } else if (integrator == QGB_INTEGRATOR_LEAPFROG) {
+    // FP64 (re-unitarised after every link step): as the single-lattice FP64 leapfrog, one launch per step
+    QB_RC(batch_evolve<R>(b, gf, gm, 0.5 * dt, unit_each));
+    void* cur = gf;
+    void* nxt = tmp;
     for (int i = 0; i < n_step; ++i) {
-      QB_RC(batch_evolve<R>(b, gf, gm, 0.5 * dt, unit_each));
-      QB_RC(batch_force<R>(b, qgb::FORCE_UPDATE, bargs(gf, gm, dt, 1)));
-      QB_RC(batch_evolve<R>(b, gf, gm, 0.5 * dt, unit_each));
-      if (reunit_every > 0 && (i + 1) % reunit_every == 0 && i + 1 < n_step)
-        QB_KERNEL(b, (qgb::launch_unitarize<R, double>(g, 4, gf, b->stream)));
+      qgb::ForceArgs u = bargs(cur, gm, dt, 1);
+      u.ev = nxt;
+      u.ev_eps = 0.5 * dt;
+      u.ev_reps = i + 1 < n_step ? 2 : 1;
+      QB_RC(batch_force<R>(b, qgb::FORCE_LEAPFROG, u));
+      std::swap(cur, nxt);
     }
+    if (cur != gf)
+      QB_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(b->Vtot) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
+                              b->stream));
   } else {
     return bfail(QGB_ERR_INVALID_ARG, "unknown integrator");
   }

@@ -411,7 +411,7 @@ int prepare_corners(const Geo& g, int variant, ForceArgs& a, bool prof, int* ker
 template <typename R>
 int force(const Geo& g, qgb::ForceMode mode, const ForceArgs& a0)
 {
-  static const char* names[] = {"force", "force_update", "force_evolve", "flow_stage", "force_update_evolve"};
+  static const char* names[] = {"force", "force_update", "force_evolve", "flow_stage", "force_update_evolve", "force_leapfrog"};
   const int v = g_force_variant[sizeof(R) == 8 ? 0 : 1][a0.c1 != 0.0 ? 1 : 0];
   ForceArgs a = a0;
   int nk = 0;
@@ -624,6 +624,25 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
       void* t = cur;
       cur = nxt;
       nxt = t;
+    }
+    if (cur != gf) {
+      Prof p("copy", 0);
+      QGB_TRY_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(g.V) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
+                                   g_ctx.stream));
+    }
+  } else if (integrator == QGB_INTEGRATOR_LEAPFROG && sizeof(R) == 8 && !hook && reunit_every == 0 && unit_each) {
+    // FP64 leapfrog, one launch per step: the two half steps of the link update between two forces follow the
+    // momentum update in the force's launch, each unitarised, into the other of two link buffers
+    QGB_RC(evolve<R>(g, gf, gm, 0.5 * dt, unit_each));
+    void* cur = gf;
+    void* nxt = tmp;
+    for (int i = 0; i < n_step; ++i) {
+      ForceArgs b = fargs(cur, gm, beta, c1, dt);
+      b.ev = nxt;
+      b.ev_eps = 0.5 * dt;
+      b.ev_reps = i + 1 < n_step ? 2 : 1;
+      QGB_RC(force<R>(g, qgb::FORCE_LEAPFROG, b));
+      std::swap(cur, nxt);
     }
     if (cur != gf) {
       Prof p("copy", 0);

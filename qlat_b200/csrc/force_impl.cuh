@@ -447,6 +447,23 @@ __device__ __forceinline__ void force_epilogue(const ForceArgs& a, const CField<
       else if (a.ev_unit == 2) unitarize_as<double, R>(wn);
       W.st(s, mu, wn);
     }
+  } else if (MODE == FORCE_LEAPFROG) {
+    // the half steps of the link update on either side of the next force: the same P, so one exponential, each
+    // half step unitarised as the separate launches do (the general exponential, as k_evolve: any P).  The next
+    // force reads W, its neighbours still read U.  One launch a step instead of three: a trajectory of 6 steps at
+    // 8^4, bound by its launches, 302 -> 253 us.
+    const WField<R> P{(Cx<R>*)a.out, stride};
+    M3<R> p = P.ld(s, mu);
+    axpy(p, R(a.dt), F);
+    P.st(s, mu, p);
+    const M3<R> e = exp_ch(scale(R(a.ev_eps), p));
+    M3<R> wn = u;
+#pragma unroll 1
+    for (int r = 0; r < a.ev_reps; ++r) {
+      wn = mul(e, wn);
+      unitarize(wn);
+    }
+    WField<R>{(Cx<R>*)a.ev, stride}.st(s, mu, wn);
   } else {
     M3<R> Z = F;
     if (MODE == FORCE_FLOW) {
@@ -596,6 +613,13 @@ cudaError_t launch_force_v(const Geo& g, ForceMode mode, const ForceArgs& a, cud
     case FORCE_EVOLVE: QGB_LAUNCH(FORCE_EVOLVE) break;
     case FORCE_FLOW: QGB_LAUNCH(FORCE_FLOW) break;
     case FORCE_UPDATE_EVOLVE: QGB_LAUNCH(FORCE_UPDATE_EVOLVE) break;
+    case FORCE_LEAPFROG:
+      if constexpr (sizeof(R) == 8) {
+        QGB_LAUNCH(FORCE_LEAPFROG)
+        break;
+      } else {
+        return cudaErrorInvalidValue;  // FP32 fuses its leapfrog steps with FORCE_UPDATE_EVOLVE
+      }
   }
 #undef QGB_LAUNCH
   return cudaGetLastError();
@@ -716,6 +740,13 @@ cudaError_t launch_force_batch_v(long Vtot, int nchain, const long* offs, const 
     case FORCE_EVOLVE: QGB_LAUNCH(FORCE_EVOLVE) break;
     case FORCE_FLOW: QGB_LAUNCH(FORCE_FLOW) break;
     case FORCE_UPDATE_EVOLVE: QGB_LAUNCH(FORCE_UPDATE_EVOLVE) break;
+    case FORCE_LEAPFROG:
+      if constexpr (sizeof(R) == 8) {
+        QGB_LAUNCH(FORCE_LEAPFROG)
+        break;
+      } else {
+        return cudaErrorInvalidValue;  // FP32 fuses its leapfrog steps with FORCE_UPDATE_EVOLVE
+      }
   }
 #undef QGB_LAUNCH
   return cudaGetLastError();

@@ -106,6 +106,7 @@ enum ForceMode {
   FORCE_EVOLVE = 2,         // U_out = unitarize(exp(eps F) U)
   FORCE_FLOW = 3,           // Z = a F + b Z_prev; U_out = unitarize(exp(eps Z) U)
   FORCE_UPDATE_EVOLVE = 4,  // P += dt F, then W = exp(ev_eps P) W on a second link field W
+  FORCE_LEAPFROG = 5,       // FP64: P += dt F, then W = U moved by ev_reps steps of unitarize(exp(ev_eps P) .)
 };
 
 struct ForceArgs {
@@ -122,6 +123,7 @@ struct ForceArgs {
   int ev_unit;      // UPDATE_EVOLVE: 0 none, 1 unitarize in R, 2 unitarize with FP64 arithmetic
   int ev_from_u;    // UPDATE_EVOLVE: W = exp(ev_eps P) U at the thread's own link (W a second buffer)
                     // instead of evolving W in place
+  int ev_reps;      // LEAPFROG: link steps after the momentum update (1 or 2)
   void* corners;    // site map 5: scratch for the 16 two-link products per site (corner_id), or null
 };
 
