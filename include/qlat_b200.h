@@ -590,7 +590,9 @@ int qgb_field_unpack_box(qgb_field* f, const int32_t lo[4], const int32_t n[4], 
  * mapping and staple evaluation (0: consecutive sites, one mu per block; 1:
  * each block takes the four links of a compact 4-d tile; 2: as 0 with
  * per-thread neighbour offsets and sign-specialised staple directions; 3: as 2
- * with SU(3) link chains carried as two rows, FP32 only -- FP64 runs 2).  The
+ * with SU(3) link chains carried as two rows, FP32 only -- FP64 runs 2; 6: as 3,
+ * and the rectangle force of FP32 trajectories and flow steps with two sites
+ * per thread in packed arithmetic).  The
  * shape is chosen per (precision, rect): by hand, or by timing them all on a
  * given gauge field. */
 int qgb_force_variant_count(int32_t* n);

@@ -118,10 +118,10 @@ int64_t g_launches = 0;  // kernels launched by this library
 // force-kernel launch variant per [precision: 0 = FP64, 1 = FP32][rect]; the
 // defaults are the fastest on B200 at 24^3 x 64 and 32^4 (FP64: 128 threads x
 // 3 blocks per SM for the plaquette force, 256 x 1 for Iwasaki; FP32, two-row
-// chains: 128 x 8 for the plaquette force, 128 x 4 for Iwasaki), so callers
-// that never run the autotuner (the reference's API has no such call) start
-// from them
-int g_force_variant[2][2] = {{6, 5}, {13, 10}};
+// chains: 128 x 8 for the plaquette force; pairs of sites for Iwasaki), so
+// callers that never run the autotuner (the reference's API has no such call)
+// start from them
+int g_force_variant[2][2] = {{6, 5}, {13, 17}};
 
 int ensure_ctx()
 {
@@ -408,15 +408,21 @@ int prepare_corners(const Geo& g, int variant, ForceArgs& a, bool prof, int* ker
   return QGB_OK;
 }
 
+const char* force_name(qgb::ForceMode mode)
+{
+  static const char* names[] = {"force",      "force_update",        "force_evolve",
+                                "flow_stage", "force_update_evolve", "force_leapfrog"};
+  return names[mode];
+}
+
 template <typename R>
 int force(const Geo& g, qgb::ForceMode mode, const ForceArgs& a0)
 {
-  static const char* names[] = {"force", "force_update", "force_evolve", "flow_stage", "force_update_evolve", "force_leapfrog"};
   const int v = g_force_variant[sizeof(R) == 8 ? 0 : 1][a0.c1 != 0.0 ? 1 : 0];
   ForceArgs a = a0;
   int nk = 0;
   QGB_RC(prepare_corners<R>(g, v, a, true, &nk));
-  Prof p(names[mode]);
+  Prof p(force_name(mode));
   QGB_TRY_CUDA(qgb::launch_force<R>(g, mode, a, v, g_ctx.stream));
   return QGB_OK;
 }
@@ -440,6 +446,51 @@ ForceArgs fargs(const void* U, void* out, double beta, double c1, double dt)
   a.dt = dt;
   a.unitarize = 1;
   return a;
+}
+
+// FP32 links, and momenta or flow fields, packed in pairs of sites for a run of force launches (force_pair.cu).
+struct PairFields {
+  qgb::PairGeo pg;
+  void *u = nullptr, *t = nullptr, *p = nullptr;  // links, a second link buffer, momenta (or Z)
+};
+
+// Whether the rectangle force of an FP32 run on lattice g goes in pairs: selected (site map 6) and possible, and
+// enough pairs to fill the GPU.  Half as many threads run twice as long, and the fields are packed before and
+// after: 8 force-gradient steps of Iwasaki at 8^4 take 0.61 ms in pairs against 0.52, at 12870 pairs (404 blocks
+// on 148 SMs of 2) 1.36 against 1.39 and the leapfrog 0.436 against 0.425, at 16^4 (32768 pairs) 2.77 against 3.00,
+// at 24^3 x 64 35.0 against 38.9.
+const long MIN_PAIRS = 16384;
+
+int use_pairs(const Geo& g, double c1, bool* yes, PairFields* f)
+{
+  int bs, minb, split, map;
+  *yes = c1 != 0.0 && qgb::force_variant_info_c(g_force_variant[1][1], &bs, &minb, &split, &map) && map == 6 &&
+         qgb::pair_geo(g, &f->pg) && f->pg.pairs >= MIN_PAIRS;
+  if (!*yes) return QGB_OK;
+  QGB_RC(get_scratch(f->pg.bytes, 71, &f->u));
+  QGB_RC(get_scratch(f->pg.bytes, 72, &f->t));
+  return get_scratch(f->pg.bytes, 73, &f->p);
+}
+
+int pair_pack(const Geo& g, const PairFields& f, const void* natural, void* packed)
+{
+  Prof p("pair_pack");
+  QGB_TRY_CUDA(qgb::launch_pair_pack(g, f.pg, natural, packed, g_ctx.stream));
+  return QGB_OK;
+}
+
+int pair_unpack(const Geo& g, const PairFields& f, const void* packed, void* natural)
+{
+  Prof p("pair_pack");
+  QGB_TRY_CUDA(qgb::launch_pair_unpack(g, f.pg, packed, natural, g_ctx.stream));
+  return QGB_OK;
+}
+
+int force_pair(const PairFields& f, qgb::ForceMode mode, const ForceArgs& a)
+{
+  Prof p(force_name(mode));
+  QGB_TRY_CUDA(qgb::launch_force_pair(f.pg, mode, a, g_ctx.stream));
+  return QGB_OK;
 }
 
 // ---- trajectories as CUDA graphs ----------------------------------------------
@@ -579,12 +630,32 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
   // force-gradient step, so gf is never read at other links; for leapfrog U is
   // gf itself, so leapfrog keeps the separate evolve).  ev_unit 2 is the
   // re-unitarisation with FP64 arithmetic due after that step.
+  // FP32 with rectangles: after the first link update the fields u, p, t go on in pairs of sites
+  bool pairs = false;
+  PairFields pf;
+  void *u = gf, *p = gm, *t = tmp;
+  if (sizeof(R) == 4 && !hook) QGB_RC(use_pairs(g, c1, &pairs, &pf));
+  auto to_pairs = [&]() -> int {
+    if (!pairs) return QGB_OK;
+    u = pf.u;
+    p = pf.p;
+    t = pf.t;
+    QGB_RC(pair_pack(g, pf, gf, u));
+    return pair_pack(g, pf, gm, p);
+  };
+  auto from_pairs = [&](const void* links) -> int {
+    QGB_RC(pair_unpack(g, pf, links, gf));
+    return pair_unpack(g, pf, p, gm);
+  };
+  auto launch = [&](qgb::ForceMode mode, const ForceArgs& a) -> int {
+    return pairs ? force_pair(pf, mode, a) : force<R>(g, mode, a);
+  };
   auto update_evolve = [&](const void* U, double h, double eps, bool reunit) -> int {
-    ForceArgs b = fargs(U, gm, beta, c1, h);
-    b.ev = gf;
+    ForceArgs b = fargs(U, p, beta, c1, h);
+    b.ev = u;
     b.ev_eps = eps;
     b.ev_unit = reunit ? 2 : unit_each;
-    return force<R>(g, qgb::FORCE_UPDATE_EVOLVE, b);
+    return launch(qgb::FORCE_UPDATE_EVOLVE, b);
   };
   if (integrator == QGB_INTEGRATOR_FORCE_GRADIENT) {
     const double lam = 0.5 * (1.0 - 1.0 / sqrt(3.0));
@@ -592,18 +663,20 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
     const double ttheta = theta * dt * dt * dt;
     const double fg_dt = 4.0 * ttheta / dt;
     QGB_RC(evolve<R>(g, gf, gm, lam * dt, unit_each));
+    QGB_RC(to_pairs());
     for (int i = 0; i < n_step; ++i) {
       const bool reunit = reunit_every > 0 && (i + 1) % reunit_every == 0 && i + 1 < n_step;
       for (int half = 0; half < 2; ++half) {
         QGB_RC(refresh());
-        ForceArgs a = fargs(gf, tmp, beta, c1, fg_dt);
+        ForceArgs a = fargs(u, t, beta, c1, fg_dt);
         a.unitarize = unit_each;
-        QGB_RC(force<R>(g, qgb::FORCE_EVOLVE, a));
+        QGB_RC(launch(qgb::FORCE_EVOLVE, a));
         if (hook_shifted) QGB_RC(refresh_field(&shifted));
         const double eps = half == 0 ? (1.0 - 2.0 * lam) * dt : (i < n_step - 1 ? 2.0 * lam : lam) * dt;
-        QGB_RC(update_evolve(tmp, 0.5 * dt, eps, half == 1 && reunit));
+        QGB_RC(update_evolve(t, 0.5 * dt, eps, half == 1 && reunit));
       }
     }
+    if (pairs) QGB_RC(from_pairs(u));
   } else if (integrator == QGB_INTEGRATOR_LEAPFROG && sizeof(R) == 4 && !hook) {
     // FP32 leapfrog with each step in one launch: the half steps of the link
     // update that meet between two force evaluations are one step of dt
@@ -611,22 +684,23 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
     // kernel, which writes the updated links into the other of two buffers
     // (gf, tmp) while its neighbours still read the current ones.
     QGB_RC(evolve<R>(g, gf, gm, 0.5 * dt, unit_each));
-    void* cur = gf;
-    void* nxt = tmp;
+    QGB_RC(to_pairs());
+    void* cur = u;
+    void* nxt = t;
     for (int i = 0; i < n_step; ++i) {
       const bool reunit = reunit_every > 0 && (i + 1) % reunit_every == 0 && i + 1 < n_step;
-      ForceArgs b = fargs(cur, gm, beta, c1, dt);
+      ForceArgs b = fargs(cur, p, beta, c1, dt);
       b.ev = nxt;
       b.ev_from_u = 1;
       b.ev_eps = i + 1 < n_step ? dt : 0.5 * dt;
       b.ev_unit = reunit ? 2 : unit_each;
-      QGB_RC(force<R>(g, qgb::FORCE_UPDATE_EVOLVE, b));
-      void* t = cur;
-      cur = nxt;
-      nxt = t;
+      QGB_RC(launch(qgb::FORCE_UPDATE_EVOLVE, b));
+      std::swap(cur, nxt);
     }
-    if (cur != gf) {
-      Prof p("copy", 0);
+    if (pairs) {
+      QGB_RC(from_pairs(cur));
+    } else if (cur != gf) {
+      Prof pc("copy", 0);
       QGB_TRY_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(g.V) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
                                    g_ctx.stream));
     }
@@ -678,9 +752,23 @@ int hamiltonian_slots(const qgb_field* gm, const qgb_field* gf, double c1, int s
 // One step of the force-gradient integrator's two force launches with
 // variant v (the shapes are timed on what the trajectories run): the shift
 // T1 = exp(eps F(U)) U, then P += dt F(T1) with T2 = exp(eps P) T2.
+// pf: those fields in pairs of sites (U in pf->u, P in pf->p; the second link
+// field is U itself), or null when the lattice cannot be packed.
 template <typename R>
-static cudaError_t fg_pair(const Geo& g, const void* U, void* T1, void* P, void* T2, double c1, int v)
+static cudaError_t fg_pair(const Geo& g, const void* U, void* T1, void* P, void* T2, double c1, int v,
+                           const PairFields* pf)
 {
+  int bs, minb, split, map;
+  qgb::force_variant_info_c(v, &bs, &minb, &split, &map);
+  if (sizeof(R) == 4 && map == 6 && pf) {
+    ForceArgs a = fargs(pf->u, pf->t, 3.0, c1, 1e-4);
+    const cudaError_t e = qgb::launch_force_pair(pf->pg, qgb::FORCE_EVOLVE, a, g_ctx.stream);
+    if (e != cudaSuccess) return e;
+    ForceArgs b = fargs(pf->t, pf->p, 3.0, c1, 1e-3);
+    b.ev = pf->u;
+    b.ev_eps = 1e-3;
+    return qgb::launch_force_pair(pf->pg, qgb::FORCE_UPDATE_EVOLVE, b, g_ctx.stream);
+  }
   ForceArgs a = fargs(U, T1, 3.0, c1, 1e-4);
   int nk = 0;
   if (prepare_corners<R>(g, v, a, false, &nk) != QGB_OK) return cudaErrorUnknown;
@@ -702,6 +790,24 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
 {
   QGB_RC(no_domain(gf, "gradient flow"));
   const Geo g = geo_of(gf);
+  bool pairs = false;
+  PairFields pf;
+  if (gf->prec == QGB_F32 && rk3) QGB_RC(use_pairs(g, c1, &pairs, &pf));
+  if (pairs) {
+    QGB_RC(pair_pack(g, pf, gf->d, pf.u));
+    auto stage = [&](const void* in, void* out, double a, double b, const void* zp, void* zo) -> int {
+      ForceArgs fa = fargs(in, out, 3.0, c1, eps);
+      fa.a = a;
+      fa.b = b;
+      fa.zp = zp;
+      fa.z = zo;
+      return force_pair(pf, qgb::FORCE_FLOW, fa);
+    };
+    QGB_RC(stage(pf.u, pf.t, 0.25, 0.0, nullptr, pf.p));
+    QGB_RC(stage(pf.t, pf.u, 8.0 / 9.0, -17.0 / 9.0, pf.p, pf.p));
+    QGB_RC(stage(pf.u, pf.t, 0.75, -1.0, pf.p, nullptr));
+    return pair_unpack(g, pf, pf.t, gf->d);
+  }
   void *T = nullptr, *Z = nullptr;
   QGB_RC(get_scratch(gf->bytes, 21, &T));
   QGB_RC(get_scratch(gf->bytes, 22, &Z));
@@ -2180,6 +2286,17 @@ int qgb_autotune_force(const qgb_field* gf, double c1, int32_t reps, int32_t* be
   QGB_RC(get_scratch(gf->bytes, 33, &T2));
   QGB_TRY_CUDA(cudaMemsetAsync(P, 0, gf->bytes, g_ctx.stream));
   QGB_TRY_CUDA(cudaMemcpyAsync(T2, gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+  // the shape that runs in pairs of sites is timed on packed copies
+  PairFields pf;
+  bool pairs = false;
+  if (gf->prec == QGB_F32 && c1 != 0.0 && qgb::pair_geo(g, &pf.pg) && pf.pg.pairs >= MIN_PAIRS) {
+    QGB_RC(get_scratch(pf.pg.bytes, 71, &pf.u));
+    QGB_RC(get_scratch(pf.pg.bytes, 72, &pf.t));
+    QGB_RC(get_scratch(pf.pg.bytes, 73, &pf.p));
+    QGB_RC(pair_pack(g, pf, gf->d, pf.u));
+    QGB_RC(pair_pack(g, pf, P, pf.p));
+    pairs = true;
+  }
   cudaEvent_t e0 = get_event(), e1 = get_event();
   const int nv = qgb::force_variant_count();
   // two interleaved passes over the shapes, the better time of each kept:
@@ -2197,8 +2314,8 @@ int qgb_autotune_force(const qgb_field* gf, double c1, int32_t reps, int32_t* be
       // the power cap, it was never faster than the two-row chains.
       if (map == 5) continue;
       auto launch = [&]() {
-        return gf->prec == QGB_F64 ? fg_pair<double>(g, gf->d, T1, P, T2, c1, v)
-                                   : fg_pair<float>(g, gf->d, T1, P, T2, c1, v);
+        return gf->prec == QGB_F64 ? fg_pair<double>(g, gf->d, T1, P, T2, c1, v, nullptr)
+                                   : fg_pair<float>(g, gf->d, T1, P, T2, c1, v, pairs ? &pf : nullptr);
       };
       QGB_TRY_CUDA(launch());
       QGB_TRY_CUDA(cudaEventRecord(e0, g_ctx.stream));

@@ -491,7 +491,9 @@ __device__ __forceinline__ void force_epilogue(const ForceArgs& a, const CField<
 // SPLIT = 1, otherwise MAP 0); MAP 3 is MAP 2 with the two-row SU(3) chains
 // (FP32; FP64 runs MAP 2); MAP 5 is MAP 3 with the staples formed from the
 // corner field of k_corners (FP32; needs ForceArgs::corners and 144 padded
-// sites < 2^31, otherwise MAP 3; FP64 runs MAP 2).
+// sites < 2^31, otherwise MAP 3; FP64 runs MAP 2); MAP 6 runs the rectangle
+// force of FP32 molecular dynamics and flow steps on pairs of sites
+// (force_pair.cu), and every other launch as MAP 3 (FP64: MAP 2).
 #define QGB_FORCE_VARIANTS(X) \
   X(0, 128, 1, 1, 0)          \
   X(1, 256, 1, 1, 0)          \
@@ -509,8 +511,9 @@ __device__ __forceinline__ void force_epilogue(const ForceArgs& a, const CField<
   X(13, 128, 8, 1, 3)         \
   X(14, 128, 4, 1, 5)         \
   X(15, 128, 3, 1, 5)         \
-  X(16, 256, 2, 1, 5)
-static const int N_FORCE_VARIANTS = 17;
+  X(16, 256, 2, 1, 5)         \
+  X(17, 128, 2, 1, 6)
+static const int N_FORCE_VARIANTS = 18;
 
 template <int BS>
 struct Tile {
@@ -586,8 +589,15 @@ __global__ void __launch_bounds__(BS, MINB) k_force(Geo g, ForceArgs a)
 template <typename R, int BS, int MINB, int SPLIT, int MAP>
 cudaError_t launch_force_v(const Geo& g, ForceMode mode, const ForceArgs& a, cudaStream_t st)
 {
-  if constexpr ((MAP == 3 || MAP == 5) && sizeof(R) == 8) {
+  if constexpr ((MAP == 3 || MAP == 5 || MAP == 6) && sizeof(R) == 8) {
     return launch_force_v<R, BS, MINB, SPLIT, 2>(g, mode, a, st);
+  } else if constexpr (MAP == 6) {
+    // 3 blocks per SM are faster (Iwasaki, 11 x 10 x 13 x 18: 1.39 against 1.56 ms for 8 force-gradient steps;
+    // 24^3 x 64: 38.9 against 40.5) unless 4 take the whole grid at once and 3 do not (8^3 x 32: 0.96 against
+    // 1.07); 148 SMs
+    const long blocks = 4 * ((work_sites(g) + 127) / 128);
+    if (blocks > 3 * 148 && blocks <= 4 * 148) return launch_force_v<R, 128, 4, 1, 3>(g, mode, a, st);
+    return launch_force_v<R, 128, 3, 1, 3>(g, mode, a, st);
   } else {
   // site map 5 reads the corner field that launch_corners filled from a.U
   if (MAP == 5 && !(a.corners && g.off == 0 && padded_sites(g.V) * 144 < 2147483647L))

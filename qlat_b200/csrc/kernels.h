@@ -134,6 +134,22 @@ struct ForceArgs {
 __host__ __device__ __forceinline__ int corner_id(int a, int b) { return 4 + 3 * a + (b < a ? b : b - 1); }
 static const int N_CORNER_FIELDS = 16;
 
+// FP32 fields packed in pairs of sites half a lattice apart (force_pair.cu).
+struct PairGeo {
+  Geo g;       // the packed field: extent half + 4 along p; its box (bl, bn) the pairs themselves
+  int p;       // the paired direction
+  int half;    // pairs along p
+  long pairs;  // pairs of sites
+  long stride; // of the site index along p
+  size_t bytes;  // one packed field of four color matrices
+};
+bool pair_geo(const Geo& g, PairGeo* out);  // false: the lattice cannot be packed
+cudaError_t launch_pair_pack(const Geo& g, const PairGeo& pg, const void* f, void* packed, cudaStream_t st);
+cudaError_t launch_pair_unpack(const Geo& g, const PairGeo& pg, const void* packed, void* f, cudaStream_t st);
+// FORCE_EVOLVE, FORCE_FLOW and FORCE_UPDATE_EVOLVE with c1 != 0 on packed fields; the link fields a launch
+// writes get their borders too.
+cudaError_t launch_force_pair(const PairGeo& pg, ForceMode mode, const ForceArgs& a, cudaStream_t st);
+
 void init_constants();  // SHA-256 and log tables into constant memory (per device)
 
 // `variant` indexes the autotuner's table of launch shapes (force_impl.cuh).

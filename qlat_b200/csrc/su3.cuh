@@ -44,7 +44,7 @@ QGB_HD M3<R> m3_zero()
 {
   M3<R> m;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) m.e[i] = cx<R>(0, 0);
+  for (int i = 0; i < 9; ++i) m.e[i] = cx<R>(R(0), R(0));
   return m;
 }
 
