@@ -194,71 +194,60 @@ __device__ __forceinline__ void staple_dir_two_row(M3<R>& S, const LinkLd<R>& L,
   }
 }
 
-template <typename R, bool RECT, int SG>
-__device__ __forceinline__ void staple_dir_fast(M3<R>& S, const LinkLd<R>& L, int s, int mu, int nu, int dmm1,
-                                                int dmp1, int dmp2, int dn1, int dn2, R cp, R cr)
+// The plaquette staple of one signed direction with full products.
+template <typename R, int SG>
+__device__ __forceinline__ void staple_dir_plaq(M3<R>& S, const LinkLd<R>& L, int s, int mu, int nu, int dmp1, int dn1)
 {
+  if (SG > 0) S = add_mul_adj(S, mul(L(nu, s), L(mu, s + dn1)), L(nu, s + dmp1));
+  else S = add_mul(S, adj_mul(L(nu, s + dn1), L(mu, s + dn1)), L(nu, s + dmp1 + dn1));
+}
+
+// Plaquette and rectangles of one signed direction with full products (FP64), every link loaded a product
+// ahead of its use; H and X are hop(x)(^+) and the next hop(x+e)(^+), loaded during the previous direction,
+// and next(H, X) loads the following direction's during this one's last two products.  At 255 registers only 8
+// warps share an SM, and without this the loads at the head of each product chain were a quarter of the
+// kernel's stalls.  Iwasaki force + momentum + link update, FP64: 24^3 x 64 2.55 -> 2.43 ms, 16^3 x 32 0.40 ->
+// 0.36 ms (128 threads, 2 blocks per SM; one block of 256 takes 2.46 and 0.37).  The plaquette force, at 168
+// registers and 12 warps, loses by it (0.80 -> 0.93 ms a flow stage at 32^4), and so does the FP32 form.
+template <typename R, int SG, typename Next>
+__device__ __forceinline__ void staple_dir_ahead(M3<R>& S, M3<R>& H, M3<R>& X, const LinkLd<R>& L, int s, int mu, int nu,
+                                                 int dmm1, int dmp1, int dmp2, int dn1, int dn2, R cp, R cr, Next next)
+{
+  M3<R> T, U01, C;
+  const M3<R> V = L(mu, s + dn2);
   if (SG > 0) {
-    const M3<R> H = L(nu, s);  // hop(x)
-    if (!RECT) {
-      S = add_mul_adj(S, mul(H, L(mu, s + dn1)), L(nu, s + dmp1));
-      return;
-    }
-    M3<R> T;
-    {  // rect1: hop(x) hop(x+e) U_mu(x+2e) back(x+2e+mu)
-      M3<R> C = mul(H, L(nu, s + dn1));
-      C = mul(C, L(mu, s + dn2));
-      C = mul_adj(C, L(nu, s + dmp1 + dn1));
-      T = scale(cr, C);
-    }
-    M3<R> U01;
-    {  // rect3: U_mu(x-mu)^+ hop(x-mu) U_mu(x-mu+e) U_mu(x+e)
-      M3<R> C = adj_mul(L(mu, s + dmm1), L(nu, s + dmm1));
-      C = mul(C, L(mu, s + dmm1 + dn1));
-      U01 = L(mu, s + dn1);
-      C = mul(C, U01);
-      axpy(T, cr, C);
-    }
-    const M3<R> B = mul(H, U01);
-    axpy(T, cp, B);
-    {  // rect2: B U_mu(x+e+mu) back(x+e+2mu) U_mu(x+mu)^+
-      M3<R> C = mul(B, L(mu, s + dmp1 + dn1));
-      C = mul_adj(C, L(nu, s + dmp2));
-      C = mul_adj(C, L(mu, s + dmp1));
-      axpy(S, cr, C);
-    }
-    S = add_mul_adj(S, T, L(nu, s + dmp1));
+    // rect1: hop(x) hop(x+e) U_mu(x+2e) back(x+2e+mu)
+    C = mul(H, X);
+    const M3<R> W = L(nu, s + dmp1 + dn1);
+    C = mul(C, V);
+    const M3<R> a = L(mu, s + dmm1), b = L(nu, s + dmm1);
+    T = scale(cr, mul_adj(C, W));
+    // rect3: U_mu(x-mu)^+ hop(x-mu) U_mu(x-mu+e) U_mu(x+e)
+    C = adj_mul(a, b);
   } else {
-    const M3<R> H = L(nu, s + dn1);  // hop(x)^+
-    if (!RECT) {
-      S = add_mul(S, adj_mul(H, L(mu, s + dn1)), L(nu, s + dmp1 + dn1));
-      return;
-    }
-    M3<R> T;
-    {  // rect1: (hop(x+e)^+ hop(x)^+)^+ U_mu(x+2e) back(x+2e+mu)
-      M3<R> C = mul(L(nu, s + dn2), H);
-      C = adj_mul(C, L(mu, s + dn2));
-      C = mul(C, L(nu, s + dmp1 + dn2));
-      T = scale(cr, C);
-    }
-    M3<R> U01;
-    {  // rect3: (hop(x-mu)^+ U_mu(x-mu))^+ U_mu(x-mu+e) U_mu(x+e)
-      M3<R> C = mul(L(nu, s + dmm1 + dn1), L(mu, s + dmm1));
-      C = adj_mul(C, L(mu, s + dmm1 + dn1));
-      U01 = L(mu, s + dn1);
-      C = mul(C, U01);
-      axpy(T, cr, C);
-    }
-    const M3<R> B = adj_mul(H, U01);
-    axpy(T, cp, B);
-    {  // rect2
-      M3<R> C = mul(B, L(mu, s + dmp1 + dn1));
-      C = mul(C, L(nu, s + dmp2 + dn1));
-      C = mul_adj(C, L(mu, s + dmp1));
-      axpy(S, cr, C);
-    }
-    S = add_mul(S, T, L(nu, s + dmp1 + dn1));
+    // rect1: (hop(x+e)^+ hop(x)^+)^+ U_mu(x+2e) back(x+2e+mu)
+    C = mul(X, H);
+    const M3<R> W = L(nu, s + dmp1 + dn2);
+    C = adj_mul(C, V);
+    const M3<R> a = L(nu, s + dmm1 + dn1), b = L(mu, s + dmm1);
+    T = scale(cr, mul(C, W));
+    // rect3: (hop(x-mu)^+ U_mu(x-mu))^+ U_mu(x-mu+e) U_mu(x+e)
+    C = mul(a, b);
   }
+  const M3<R> d = L(mu, s + dmm1 + dn1);
+  U01 = L(mu, s + dn1);
+  C = SG > 0 ? mul(C, d) : adj_mul(C, d);
+  axpy(T, cr, mul(C, U01));
+  const M3<R> B = SG > 0 ? mul(H, U01) : adj_mul(H, U01);
+  axpy(T, cp, B);
+  // rect2: B U_mu(x+e+mu) back(x+e+2mu) U_mu(x+mu)^+
+  C = mul(B, L(mu, s + dmp1 + dn1));
+  C = SG > 0 ? mul_adj(C, L(nu, s + dmp2)) : mul(C, L(nu, s + dmp2 + dn1));
+  const M3<R> K = SG > 0 ? L(nu, s + dmp1) : L(nu, s + dmp1 + dn1);
+  C = mul_adj(C, L(mu, s + dmp1));
+  next(H, X);
+  axpy(S, cr, C);
+  S = SG > 0 ? add_mul_adj(S, T, K) : add_mul(S, T, K);
 }
 
 // ------------------------------------------------------------------------
@@ -396,6 +385,28 @@ __device__ __forceinline__ M3<R> staple_sum_fast(const Cx<R>* U, const Geo& g, i
   const int xm = sel4(x.c, mu), Lm = sel4(g.d, mu), sm = sel4(st, mu);
   const int dmm1 = nb_delta(xm, -1, Lm, sm), dmp1 = nb_delta(xm, 1, Lm, sm), dmp2 = nb_delta(xm, 2, Lm, sm);
   M3<R> S = m3_zero<R>();
+  if constexpr (RECT && !TWO) {
+    auto off = [&](int k, int a) { return nb_delta(sel4(x.c, k), a, sel4(g.d, k), sel4(st, k)); };
+    int nu = (mu + 1) & 3;
+    M3<R> H = L(nu, s), X = L(nu, s + off(nu, 1));
+#pragma unroll 1
+    for (int i = 1; i < 4; ++i) {
+      nu = (mu + i) & 3;
+      const int m1 = off(nu, -1), m2 = off(nu, -2);
+      staple_dir_ahead<R, 1>(S, H, X, L, s, mu, nu, dmm1, dmp1, dmp2, off(nu, 1), off(nu, 2), cp, cr,
+                             [&](M3<R>& h, M3<R>& y) {
+                               h = L(nu, s + m1);
+                               y = L(nu, s + m2);
+                             });
+      const int n2 = (mu + (i < 3 ? i + 1 : 1)) & 3;  // after the last direction a load that nothing uses
+      const int o2 = off(n2, 1);
+      staple_dir_ahead<R, -1>(S, H, X, L, s, mu, nu, dmm1, dmp1, dmp2, m1, m2, cp, cr, [&](M3<R>& h, M3<R>& y) {
+        h = L(n2, s);
+        y = L(n2, s + o2);
+      });
+    }
+    return S;
+  }
 #pragma unroll 1
   for (int i = 1; i < 4; ++i) {
     const int nu = (mu + i) & 3;
@@ -406,10 +417,8 @@ __device__ __forceinline__ M3<R> staple_sum_fast(const Cx<R>* U, const Geo& g, i
       staple_dir_two_row<R, RECT, -1>(S, L, s, mu, nu, dmm1, dmp1, dmp2, nb_delta(xn, -1, Ln, sn),
                                               nb_delta(xn, -2, Ln, sn), cp, cr);
     } else {
-      staple_dir_fast<R, RECT, 1>(S, L, s, mu, nu, dmm1, dmp1, dmp2, nb_delta(xn, 1, Ln, sn),
-                                          nb_delta(xn, 2, Ln, sn), cp, cr);
-      staple_dir_fast<R, RECT, -1>(S, L, s, mu, nu, dmm1, dmp1, dmp2, nb_delta(xn, -1, Ln, sn),
-                                           nb_delta(xn, -2, Ln, sn), cp, cr);
+      staple_dir_plaq<R, 1>(S, L, s, mu, nu, dmp1, nb_delta(xn, 1, Ln, sn));
+      staple_dir_plaq<R, -1>(S, L, s, mu, nu, dmp1, nb_delta(xn, -1, Ln, sn));
     }
   }
   if (!RECT) S = scale(cp, S);
