@@ -82,9 +82,10 @@ int qgb_field_create(qgb_field** out, const int32_t total_site[4], int32_t multi
  * run_hmc_pure_gauge, hmc.pyx:190-216, builds a link copy and a momentum field
  * every trajectory). */
 int qgb_field_destroy(qgb_field* f);
-/* Frees the pooled storage of destroyed fields (qgb_field_create also does
- * this by itself when cudaMalloc runs out of memory); writes the bytes freed
- * when released is not NULL. */
+/* Frees the pooled storage of destroyed fields and the checkpoints and stage
+ * fields that the flow adjoint keeps for its next call (qgb_field_create also
+ * does this by itself when cudaMalloc runs out of memory); writes the bytes
+ * freed when released is not NULL. */
 int qgb_field_pool_release(int64_t* released);
 int qgb_field_info(const qgb_field* f, int32_t total_site[4], int32_t* multiplicity, int32_t* kind,
                    int32_t* precision);

@@ -267,6 +267,22 @@ int get_scratch(size_t bytes, int tag, void** out)
   return QGB_OK;
 }
 
+// the flow adjoint's checkpoints and stage fields (no recorded graph uses them)
+void release_adjoint_scratch(int64_t* released)
+{
+  for (auto it = g_ctx.scratch.begin(); it != g_ctx.scratch.end();) {
+    if (it->first.second < 100 || it->first.second >= 0x7A000) {  // (the other units' tags start there)
+      ++it;
+      continue;
+    }
+    for (void* p : it->second) {
+      cudaFree(p);
+      if (released) *released += (int64_t)it->first.first;
+    }
+    it = g_ctx.scratch.erase(it);
+  }
+}
+
 void release_field_pool()
 {
   for (auto& kv : g_ctx.field_pool)
@@ -837,19 +853,93 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
 
 // ---- flow adjoint ------------------------------------------------------------
 
+// Scratch of the adjoint: the states at the checkpoints (100 + c), the links
+// before each step of a segment (1000 + j) and its stage fields (2000 + 5 j + k:
+// the links after stages 1 and 2, the three stages' Z).  qgb_field_pool_release
+// gives it back.
+const int ADJ_CHECKPOINT = 100, ADJ_LINKS = 1000, ADJ_STAGES = 100000;
+
+// Stage fields kept between a flow's forward pass and its pull-back: at most this much (40 steps at 16^4 in FP64
+// are 7.0 GiB; keeping them saves the second forward pass, 31.5 -> 24.5 ms a gradient).
+const size_t ADJ_KEEP = (size_t)8 << 30;
+
+// Whether every step of the flow can keep its stage fields, so that nothing is recomputed: they fit the bound
+// and the device's free memory (with 2 GiB to spare), or are there already.
+static bool adj_keep_all(size_t bytes, int steps)
+{
+  if (steps < 1 || (size_t)5 * steps * bytes > ADJ_KEEP) return false;
+  auto have = [&](int tag) {
+    auto it = g_ctx.scratch.find(std::make_pair(bytes, tag));
+    return it != g_ctx.scratch.end() && !it->second.empty();
+  };
+  size_t need = 0;
+  for (int j = 0; j < steps; ++j) {
+    if (!have(ADJ_LINKS + j)) need += bytes;
+    for (int k = 0; k < 5; ++k)
+      if (!have(ADJ_STAGES + 5 * j + k)) need += bytes;
+  }
+  if (need == 0) return true;
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  return free_bytes >= need + ((size_t)2 << 30);
+}
+
+// One RK3 step in -> out, keeping its stage fields k: the links after stages 1
+// and 2 and the stages' Z.
+template <typename R>
+static int flow_step_kept(const Geo& g, double eps, double c1, const void* in, void* out, void* const* k)
+{
+  auto stage = [&](const void* from, void* to, double a, double b, const void* zp, void* zo) -> int {
+    ForceArgs fa = fargs(from, to, 3.0, c1, eps);
+    fa.a = a;
+    fa.b = b;
+    fa.zp = zp;
+    fa.z = zo;
+    return force<R>(g, qgb::FORCE_FLOW, fa);
+  };
+  QGB_RC(stage(in, k[0], 0.25, 0.0, nullptr, k[2]));
+  QGB_RC(stage(k[0], k[1], 8.0 / 9.0, -17.0 / 9.0, k[2], k[3]));
+  return stage(k[1], out, 0.75, -1.0, k[3], k[4]);
+}
+
+// The flow of gf into `out`, keeping every step's links and stage fields (adj_keep_all).
+template <typename R>
+static int flow_kept(const qgb_field* gf, double eps, double c1, int steps, void* out)
+{
+  const Geo g = geo_of(gf);
+  std::vector<void*> w(steps + 1), k((size_t)5 * steps);
+  for (int j = 0; j < steps; ++j) QGB_RC(get_scratch(gf->bytes, ADJ_LINKS + j, &w[j]));
+  for (int j = 0; j < 5 * steps; ++j) QGB_RC(get_scratch(gf->bytes, ADJ_STAGES + j, &k[j]));
+  w[steps] = out;
+  QGB_TRY_CUDA(cudaMemcpyAsync(w[0], gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+  for (int j = 0; j < steps; ++j) QGB_RC(flow_step_kept<R>(g, eps, c1, w[j], w[j + 1], &k[(size_t)5 * j]));
+  return QGB_OK;
+}
+
+// What the forward flow has left for the pull-back.
+enum FlowKept { FLOW_KEPT_NONE, FLOW_KEPT_CHECKPOINTS, FLOW_KEPT_STAGES };
+
 // Pull a cotangent back through RK3 flow steps (adjoint.cu): checkpoints every
 // `every` steps, each segment recomputed forward, each step's three stages
-// recomputed with their Z fields, then pulled back stage by stage.
+// recomputed with their Z fields, then pulled back stage by stage.  When every
+// step can keep its stage fields there is one segment, and none of it is
+// recomputed if the caller's forward flow has left them (FLOW_KEPT_STAGES).
 template <typename R>
 static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, int every, const void* lam_in,
-                         void* grad, bool cps_ready = false)
+                         void* grad, FlowKept kept_by_flow = FLOW_KEPT_NONE)
 {
   const Geo g = geo_of(gf);
   const size_t bytes = gf->bytes;
-  const int ncp = (steps + every - 1) / every;
+  const bool keep_all = kept_by_flow == FLOW_KEPT_STAGES ||
+                        (kept_by_flow == FLOW_KEPT_NONE && adj_keep_all(bytes, steps));
+  if (keep_all) every = steps;
+  const int ncp = keep_all ? 0 : (steps + every - 1) / every;
   std::vector<void*> cps(ncp), wst(every);
-  for (int i = 0; i < ncp; ++i) QGB_RC(get_scratch(bytes, 100 + i, &cps[i]));
-  for (int i = 0; i < every; ++i) QGB_RC(get_scratch(bytes, 1000 + i, &wst[i]));
+  for (int i = 0; i < ncp; ++i) QGB_RC(get_scratch(bytes, ADJ_CHECKPOINT + i, &cps[i]));
+  for (int i = 0; i < every; ++i) QGB_RC(get_scratch(bytes, ADJ_LINKS + i, &wst[i]));
   void *W1, *W2, *Wx, *Z0, *Z1, *Z2, *lam, *laml, *mua, *mub;
   QGB_RC(get_scratch(bytes, 41, &W1));
   QGB_RC(get_scratch(bytes, 42, &W2));
@@ -861,35 +951,22 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
   QGB_RC(get_scratch(bytes, 48, &laml));
   QGB_RC(get_scratch(bytes, 49, &mua));
   QGB_RC(get_scratch(bytes, 50, &mub));
-  auto stage = [&](const void* in, void* out, double a, double b, const void* zp, void* zo) -> int {
-    ForceArgs fa = fargs(in, out, 3.0, c1, eps);
-    fa.a = a;
-    fa.b = b;
-    fa.zp = zp;
-    fa.z = zo;
-    return force<R>(g, qgb::FORCE_FLOW, fa);
-  };
-  // one RK3 step in -> out, keeping its stage fields w1, w2 (links after
-  // stages 1, 2) and z0, z1, z2 (the stages' Z)
-  auto step_into = [&](const void* in, void* out, void* w1, void* w2, void* z0, void* z1, void* z2) -> int {
-    QGB_RC(stage(in, w1, 0.25, 0.0, nullptr, z0));
-    QGB_RC(stage(w1, w2, 8.0 / 9.0, -17.0 / 9.0, z0, z1));
-    QGB_RC(stage(w2, out, 0.75, -1.0, z1, z2));
-    return QGB_OK;
-  };
-  auto step = [&](const void* in, void* out) -> int { return step_into(in, out, W1, W2, Z0, Z1, Z2); };
+  void* const one[5] = {W1, W2, Z0, Z1, Z2};
+  auto step = [&](const void* in, void* out) -> int { return flow_step_kept<R>(g, eps, c1, in, out, one); };
   // When the five stage fields of every step of a segment fit in 4 GiB, the
   // segment's recomputation keeps them, and the pull-back reads them instead
   // of recomputing each step a second time.
-  const bool keep = (size_t)5 * every * bytes <= ((size_t)4 << 30);
+  const bool keep = keep_all || (size_t)5 * every * bytes <= ((size_t)4 << 30);
   std::vector<void*> kept;
   if (keep) {
     kept.resize((size_t)5 * every);
-    for (int i = 0; i < 5 * every; ++i) QGB_RC(get_scratch(bytes, 2000 + i, &kept[i]));
+    for (int i = 0; i < 5 * every; ++i) QGB_RC(get_scratch(bytes, ADJ_STAGES + i, &kept[i]));
   }
   // forward pass: checkpoints (the states after 0, every, 2 every, ... steps
-  // in the scratch buffers 100 + c; cps_ready: the caller's forward flow
-  // already left them there)
+  // in the scratch buffers ADJ_CHECKPOINT + c), unless the caller's forward
+  // flow already left them there
+  if (keep_all && kept_by_flow == FLOW_KEPT_NONE) QGB_RC(flow_kept<R>(gf, eps, c1, steps, Wx));
+  const bool cps_ready = keep_all || kept_by_flow == FLOW_KEPT_CHECKPOINTS;
   if (!cps_ready) QGB_TRY_CUDA(cudaMemcpyAsync(cps[0], gf->d, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   for (int c = 1; c < ncp && !cps_ready; ++c) {
     QGB_TRY_CUDA(cudaMemcpyAsync(Wx, cps[c - 1], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
@@ -901,15 +978,15 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
   }
   QGB_TRY_CUDA(cudaMemcpyAsync(lam, lam_in, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   // backward pass
-  for (int c = ncp - 1; c >= 0; --c) {
+  for (int c = keep_all ? 0 : ncp - 1; c >= 0; --c) {
     const int s0 = c * every, s1 = (s0 + every < steps) ? s0 + every : steps;
-    QGB_TRY_CUDA(cudaMemcpyAsync(wst[0], cps[c], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     const int n = s1 - s0;
-    if (keep) {
-      for (int j = 0; j < n; ++j) {
-        void** k = &kept[(size_t)5 * j];
-        QGB_RC(step_into(wst[j], j + 1 < n ? wst[j + 1] : Wx, k[0], k[1], k[2], k[3], k[4]));
-      }
+    if (!keep_all) QGB_TRY_CUDA(cudaMemcpyAsync(wst[0], cps[c], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+    if (keep_all) {
+      // all there already
+    } else if (keep) {
+      for (int j = 0; j < n; ++j)
+        QGB_RC(flow_step_kept<R>(g, eps, c1, wst[j], j + 1 < n ? wst[j + 1] : Wx, &kept[(size_t)5 * j]));
     } else {
       for (int j = 1; j < n; ++j) QGB_RC(step(wst[j - 1], wst[j]));
     }
@@ -1112,9 +1189,11 @@ int qgb_field_create(qgb_field** out, const int32_t total_site[4], int32_t multi
     g_ctx.field_pool_bytes -= f->bytes;
   } else {
     e = cudaMalloc(&f->d, f->bytes);
-    if (e == cudaErrorMemoryAllocation && g_ctx.field_pool_bytes > 0) {
+    if (e == cudaErrorMemoryAllocation) {
       cudaGetLastError();
+      cudaStreamSynchronize(g_ctx.stream);
       release_field_pool();
+      release_adjoint_scratch(nullptr);
       e = cudaMalloc(&f->d, f->bytes);
     }
   }
@@ -1155,6 +1234,7 @@ int qgb_field_pool_release(int64_t* released)
   if (released) *released = (int64_t)g_ctx.field_pool_bytes;
   if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
   release_field_pool();
+  release_adjoint_scratch(released);
   return QGB_OK;
 }
 
@@ -2133,17 +2213,24 @@ int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, 
   void *V = nullptr, *lamN = nullptr;
   QGB_RC(get_scratch(gf->bytes, 61, &V));
   QGB_RC(get_scratch(gf->bytes, 62, &lamN));
-  // flowed field V_t, keeping the adjoint's checkpoints on the way (the
-  // states after 0, every, 2 every, ... steps, in the scratch buffers that
-  // flow_vjp_impl reads)
+  // flowed field V_t, keeping on the way what flow_vjp_impl reads: every step's
+  // links and stage fields if they fit, or the checkpoints (the states after 0,
+  // every, 2 every, ... steps)
+  const bool stages = adj_keep_all(gf->bytes, steps);
   const int every = steps > 0 ? (checkpoint_every < steps ? checkpoint_every : steps) : 1;
-  QGB_TRY_CUDA(cudaMemcpyAsync(V, gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   qgb_field_s fv = *gf;
   fv.d = V;
-  for (int i = 0; i < steps; ++i) {
+  if (stages) {
+    QGB_RC(no_domain(gf, "gradient flow"));
+    if (gf->prec == QGB_F64) QGB_RC(flow_kept<double>(gf, epsilon, c1, steps, V));
+    else QGB_RC(flow_kept<float>(gf, epsilon, c1, steps, V));
+  } else {
+    QGB_TRY_CUDA(cudaMemcpyAsync(V, gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+  }
+  for (int i = 0; i < steps && !stages; ++i) {
     if (i % every == 0) {
       void* cp = nullptr;
-      QGB_RC(get_scratch(gf->bytes, 100 + i / every, &cp));
+      QGB_RC(get_scratch(gf->bytes, ADJ_CHECKPOINT + i / every, &cp));
       QGB_TRY_CUDA(cudaMemcpyAsync(cp, fv.d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     }
     QGB_RC(flow_step(&fv, epsilon, c1, true));
@@ -2167,8 +2254,9 @@ int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, 
     QGB_TRY_CUDA(cudaMemcpyAsync(grad->d, lamN, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     return QGB_OK;
   }
-  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, every, lamN, grad->d, true);
-  return flow_vjp_impl<float>(gf, epsilon, c1, steps, every, lamN, grad->d, true);
+  const FlowKept kept = stages ? FLOW_KEPT_STAGES : FLOW_KEPT_CHECKPOINTS;
+  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, every, lamN, grad->d, kept);
+  return flow_vjp_impl<float>(gf, epsilon, c1, steps, every, lamN, grad->d, kept);
 }
 
 int qgb_set_anti_hermitian_matrix_from_basis(qgb_field* fc, const qgb_field* basis)
