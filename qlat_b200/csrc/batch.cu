@@ -189,14 +189,15 @@ int batch_md(qgb_batch_s* b, void* gf, void* gm, void* tmp, int n_step, double m
   return QGB_OK;
 }
 
-// Per-chain Hamiltonian pieces of (gm, gf0) into d_sums[slot * n ...]: gm, plaq, rect.
-int batch_hamiltonian(qgb_batch_s* b, int slot)
+// Per-chain Hamiltonian pieces of (P, gf0) into d_sums[slot * n ...]: gm, plaq, rect; P are the momenta in
+// precision R.  With copies the same passes write the FP32 copies gm32 and gf32.
+template <typename R>
+int batch_hamiltonian(qgb_batch_s* b, int slot, const void* P, bool copies)
 {
-  QB_KERNEL(b, qgb::launch_site_values_batch<double>(b->Vtot, b->n, b->d_offs, b->d_chains, 0, 0, b->gm, b->d_vals,
-                                                b->stream));
+  QB_KERNEL(b, qgb::launch_batch_kinetic<R>(b->Vtot, P, copies ? b->gm32 : nullptr, b->d_vals, b->stream));
   QB_KERNEL(b, qgb::launch_segment_sum(b->n, b->d_offs, b->d_vals, b->d_sums + (long)slot * b->n, b->stream));
-  QB_KERNEL(b, qgb::launch_site_values_batch<double>(b->Vtot, b->n, b->d_offs, b->d_chains, 1, b->rect ? 1 : 0, b->gf0,
-                                                b->d_vals, b->stream));
+  QB_KERNEL(b, qgb::launch_batch_action(b->Vtot, b->n, b->d_offs, b->d_chains, b->rect ? 1 : 0, b->gf0,
+                                        copies ? b->gf32 : nullptr, b->d_vals, b->stream));
   QB_KERNEL(b, qgb::launch_segment_sum(b->n, b->d_offs, b->d_vals, b->d_sums + (long)(slot + 1) * b->n, b->stream));
   if (b->rect)
     QB_KERNEL(b, qgb::launch_segment_sum(b->n, b->d_offs, b->d_vals + b->Vtot, b->d_sums + (long)(slot + 2) * b->n,
@@ -211,25 +212,22 @@ int enqueue_trajectory(qgb_batch_s* b, int n_step, double md_time, int integrato
 {
   b->kernels = 0;
   const size_t bytes64 = (size_t)qgb::padded_sites(b->Vtot) * 72 * sizeof(double);
-  const long n = qgb::padded_sites(b->Vtot) * 72;
   qgb::Geo g;
   g.d[0] = g.d[1] = g.d[2] = g.d[3] = 1;
   g.V = b->Vtot;
   QB_CUDA(cudaMemcpyAsync(b->gf0, b->gf, bytes64, cudaMemcpyDeviceToDevice, b->stream));
   QB_KERNEL(b, qgb::launch_rand_momentum_batch<double>(b->Vtot, b->n, b->d_offs, b->d_rs, 1.0, b->gm, b->d_ambiguous,
                                                   b->stream));
-  QB_RC(batch_hamiltonian(b, 0));
+  QB_RC(batch_hamiltonian<double>(b, 0, b->gm, mixed != 0));
   if (mixed) {
-    QB_KERNEL(b, (qgb::launch_convert<double, float>(n, b->gf0, b->gf32, b->stream)));
-    QB_KERNEL(b, (qgb::launch_convert<double, float>(n, b->gm, b->gm32, b->stream)));
     QB_RC(batch_md<float>(b, b->gf32, b->gm32, b->tmp32, n_step, md_time, integrator, reunit > 0 ? 0 : 1, reunit));
-    QB_KERNEL(b, (qgb::launch_convert<float, double>(n, b->gf32, b->gf0, b->stream)));
-    QB_KERNEL(b, (qgb::launch_convert<float, double>(n, b->gm32, b->gm, b->stream)));
+    QB_KERNEL(b, qgb::launch_unitarize_to_f64(g, b->gf32, b->gf0, b->stream));
+    QB_RC(batch_hamiltonian<float>(b, 3, b->gm32, false));
   } else {
     QB_RC(batch_md<double>(b, b->gf0, b->gm, b->tmp, n_step, md_time, integrator, 1, 0));
+    QB_KERNEL(b, (qgb::launch_unitarize<double, double>(g, 4, b->gf0, b->stream)));
+    QB_RC(batch_hamiltonian<double>(b, 3, b->gm, false));
   }
-  QB_KERNEL(b, (qgb::launch_unitarize<double, double>(g, 4, b->gf0, b->stream)));
-  QB_RC(batch_hamiltonian(b, 3));
   QB_CUDA(cudaMemcpyAsync(b->h_sums, b->d_sums, 6 * b->n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
   return QGB_OK;
 }
@@ -455,8 +453,7 @@ int qgb_batch_accept(qgb_batch* b, const int32_t* flags)
 int qgb_batch_plaq(qgb_batch* b, double* plaq)
 {
   if (!b || !plaq) return bfail(QGB_ERR_INVALID_ARG, "qgb_batch_plaq: null argument");
-  QB_CUDA(qgb::launch_site_values_batch<double>(b->Vtot, b->n, b->d_offs, b->d_chains, 1, 0, b->gf, b->d_vals,
-                                                b->stream));
+  QB_CUDA(qgb::launch_batch_action(b->Vtot, b->n, b->d_offs, b->d_chains, 0, b->gf, nullptr, b->d_vals, b->stream));
   QB_CUDA(qgb::launch_segment_sum(b->n, b->d_offs, b->d_vals, b->d_sums + 6L * b->n, b->stream));
   QB_CUDA(cudaMemcpyAsync(b->h_sums + 6L * b->n, b->d_sums + 6L * b->n, b->n * sizeof(double), cudaMemcpyDeviceToHost,
                           b->stream));

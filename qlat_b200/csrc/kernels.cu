@@ -671,24 +671,101 @@ __global__ void __launch_bounds__(128) k_hot_start_batch(long Vtot, int nchain, 
   if (amb) atomicAdd(ambiguous, 1);
 }
 
-// Site values for the per-chain Hamiltonians: what = 0: sum_mu -tr(P^2)/2 from
-// P into vals[sg]; what = 1: plaquette sum (vals[sg]) and, if rect, rectangle
-// sum (vals[Vtot + sg]) from U.
+// Site values for the per-chain Hamiltonians.
+
+// vals[sg] = sum_mu -tr(P^2)/2, and with COPY the momenta converted to RO into Q in the same pass (padded sites
+// included, with the zeros of P's).  Memory-bound: 1.69 M sites (256 chains of 4^4 to 12^4), 0.21 ms with the copy and
+// 0.05 ms from FP32.
+template <typename RI, typename RO, bool COPY>
+__global__ void __launch_bounds__(256) k_batch_kinetic(long Vtot, const Cx<RI>* P, Cx<RO>* Q, double* vals)
+{
+  const long sg = (long)blockIdx.x * 256 + threadIdx.x;
+  if (sg >= padded_sites(Vtot)) return;
+  const CField<RI> Pf{P, Vtot};
+  double v = 0.0;
+#pragma unroll 1
+  for (int mu = 0; mu < 4; ++mu) {
+    const M3<RI> p = Pf.ld(sg, mu);
+    M3<double> d;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) d.e[k] = cx<double>((double)p.e[k].re, (double)p.e[k].im);
+    if (COPY) {
+      M3<RO> q;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) q.e[k] = cx<RO>((RO)p.e[k].re, (RO)p.e[k].im);
+      WField<RO>{Q, Vtot}.st(sg, mu, q);
+    }
+    v += neg_half_tr_square(d);
+  }
+  if (sg < Vtot) vals[sg] = v;
+}
+
+// Plaquette sums into vals[sg] and, with RECT, rectangle sums into vals[Vtot + sg], as k_action_corners within
+// each site's chain (8 products per plane instead of 10 from 64-bit index walks); with copy != nullptr also the
+// links in FP32 (padded sites included).
+template <bool RECT>
+__global__ void __launch_bounds__(256, RECT ? 1 : 2)
+    k_batch_action(long Vtot, int nchain, const long* __restrict__ offs, const ChainInfo* __restrict__ chains,
+                   const Cx<double>* U, Cx<float>* copy, double* vals)
+{
+  const long sg = (long)blockIdx.x * 256 + threadIdx.x;
+  if (copy != nullptr && sg < padded_sites(Vtot)) {
+    const CField<double> Uf{U, Vtot};
+#pragma unroll 1
+    for (int mu = 0; mu < 4; ++mu) {
+      const M3<double> u = Uf.ld(sg, mu);
+      M3<float> c;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) c.e[k] = cx<float>((float)u.e[k].re, (float)u.e[k].im);
+      WField<float>{copy, Vtot}.st(sg, mu, c);
+    }
+  }
+  if (sg >= Vtot) return;
+  const Geo g = chain_geo(chains[chain_of(offs, nchain, sg)]);
+  const Coord x = coord_of(g, sg - g.off);
+  const LinkLd<double> L{U, (int)site_blocks(Vtot)};
+  const int si = (int)sg;
+  const int st[4] = {1, g.d[0], g.d[0] * g.d[1], g.d[0] * g.d[1] * g.d[2]};
+  int d1[4], d2[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    d1[k] = nb_delta(x.c[k], 1, g.d[k], st[k]);
+    d2[k] = nb_delta(x.c[k], 2, g.d[k], st[k]);
+  }
+  double sp = 0.0, sr = 0.0;
+#pragma unroll 1
+  for (int p = 0; p < 6; ++p) {
+    const int a = p < 3 ? 0 : (p < 5 ? 1 : 2);
+    const int b = p < 3 ? p + 1 : (p < 5 ? p - 1 : 3);
+    const int a1 = sel4(d1, a), b1 = sel4(d1, b);
+    const M3<double> ua = L(a, si), ub = L(b, si);
+    const M3<double> Pa = mul(ua, L(b, si + a1));
+    const M3<double> Pb = mul(ub, L(a, si + b1));
+    sp += re_tr_mul_adj(Pa, Pb) - 3.0;
+    if (RECT) {
+      {
+        const M3<double> A = mul(mul(ua, L(a, si + a1)), L(b, si + sel4(d2, a)));
+        sr += re_tr_mul_adj(A, mul(Pb, L(a, si + a1 + b1))) - 3.0;
+      }
+      {
+        const M3<double> A = mul(mul(ub, L(b, si + b1)), L(a, si + sel4(d2, b)));
+        sr += re_tr_mul_adj(A, mul(Pa, L(b, si + a1 + b1))) - 3.0;
+      }
+    }
+  }
+  vals[sg] = sp;
+  if (RECT) vals[Vtot + sg] = sr;
+}
+
+// The action sums where 32-bit link offsets would overflow.
 template <typename R>
-__global__ void __launch_bounds__(128) k_site_values_batch(long Vtot, int nchain, const long* __restrict__ offs,
-                                                           const ChainInfo* __restrict__ chains, int what, int rect,
-                                                           const Cx<R>* F, double* vals)
+__global__ void __launch_bounds__(128) k_batch_action_large(long Vtot, int nchain, const long* __restrict__ offs,
+                                                            const ChainInfo* __restrict__ chains, int rect,
+                                                            const Cx<R>* F, double* vals)
 {
   const long sg = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (sg >= Vtot) return;
   const CField<R> Ff{F, Vtot};
-  if (what == 0) {
-    double v = 0.0;
-#pragma unroll
-    for (int mu = 0; mu < 4; ++mu) v += neg_half_tr_square(Ff.ld(sg, mu));
-    vals[sg] = v;
-    return;
-  }
   const int c = chain_of(offs, nchain, sg);
   const Geo g = chain_geo(chains[c]);
   const Coord x = coord_of(g, sg - g.off);
@@ -768,12 +845,28 @@ cudaError_t launch_hot_start_batch(long Vtot, int nchain, const long* offs, cons
   return cudaGetLastError();
 }
 
-template <typename R>
-cudaError_t launch_site_values_batch(long Vtot, int nchain, const long* offs, const ChainInfo* chains, int what,
-                                     int rect, const void* F, double* vals, cudaStream_t st)
+template <typename RI>
+cudaError_t launch_batch_kinetic(long Vtot, const void* P, void* copy_f32, double* vals, cudaStream_t st)
 {
-  k_site_values_batch<R><<<(unsigned)((Vtot + 127) / 128), 128, 0, st>>>(Vtot, nchain, offs, chains, what, rect,
-                                                                        (const Cx<R>*)F, vals);
+  const unsigned grid = (unsigned)((padded_sites(Vtot) + 255) / 256);
+  if (copy_f32) k_batch_kinetic<RI, float, true><<<grid, 256, 0, st>>>(Vtot, (const Cx<RI>*)P, (Cx<float>*)copy_f32, vals);
+  else k_batch_kinetic<RI, float, false><<<grid, 256, 0, st>>>(Vtot, (const Cx<RI>*)P, nullptr, vals);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_batch_action(long Vtot, int nchain, const long* offs, const ChainInfo* chains, int rect,
+                                const void* U, void* copy_f32, double* vals, cudaStream_t st)
+{
+  const Cx<double>* u = (const Cx<double>*)U;
+  Cx<float>* c = (Cx<float>*)copy_f32;
+  if (padded_sites(Vtot) * 36 < 2147483647L) {
+    const unsigned grid = (unsigned)((padded_sites(Vtot) + 255) / 256);
+    if (rect) k_batch_action<true><<<grid, 256, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
+    else k_batch_action<false><<<grid, 256, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
+    return cudaGetLastError();
+  }
+  k_batch_action_large<double><<<(unsigned)((Vtot + 127) / 128), 128, 0, st>>>(Vtot, nchain, offs, chains, rect, u, vals);
+  if (c != nullptr) return launch_convert<double, float>(padded_sites(Vtot) * 72, U, c, st);
   return cudaGetLastError();
 }
 
@@ -796,10 +889,8 @@ template cudaError_t launch_rand_momentum_batch<double>(long, int, const long*, 
                                                         cudaStream_t);
 template cudaError_t launch_hot_start_batch<double>(long, int, const long*, const uint32_t*, double, int, void*, int*,
                                                     cudaStream_t);
-template cudaError_t launch_site_values_batch<double>(long, int, const long*, const ChainInfo*, int, int, const void*,
-                                                      double*, cudaStream_t);
-template cudaError_t launch_site_values_batch<float>(long, int, const long*, const ChainInfo*, int, int, const void*,
-                                                     double*, cudaStream_t);
+template cudaError_t launch_batch_kinetic<double>(long, const void*, void*, double*, cudaStream_t);
+template cudaError_t launch_batch_kinetic<float>(long, const void*, void*, double*, cudaStream_t);
 template cudaError_t launch_accept_batch<double>(long, int, const long*, const int*, void*, const void*, cudaStream_t);
 
 // ------------------------------------------------------------------------

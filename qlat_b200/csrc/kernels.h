@@ -243,9 +243,12 @@ cudaError_t launch_rand_momentum_batch(long Vtot, int nchain, const long* offs, 
 template <typename R>
 cudaError_t launch_hot_start_batch(long Vtot, int nchain, const long* offs, const uint32_t* rs24, double sigma,
                                    int n_step, void* U, int* ambiguous, cudaStream_t st);
-template <typename R>
-cudaError_t launch_site_values_batch(long Vtot, int nchain, const long* offs, const ChainInfo* chains, int what,
-                                     int rect, const void* F, double* vals, cudaStream_t st);
+// Per-site kinetic values of all chains' momenta, and of their links plaquette (vals[sg]) and rectangle
+// (vals[Vtot + sg]) sums; with copy_f32 also the FP32 copy of the field.
+template <typename RI>
+cudaError_t launch_batch_kinetic(long Vtot, const void* P, void* copy_f32, double* vals, cudaStream_t st);
+cudaError_t launch_batch_action(long Vtot, int nchain, const long* offs, const ChainInfo* chains, int rect,
+                                const void* U, void* copy_f32, double* vals, cudaStream_t st);
 cudaError_t launch_segment_sum(int nchain, const long* offs, const double* vals, double* out, cudaStream_t st);
 template <typename R>
 cudaError_t launch_accept_batch(long Vtot, int nchain, const long* offs, const int* flags, void* dst, const void* src,
