@@ -477,15 +477,29 @@ struct PairFields {
 // at 24^3 x 64 35.0 against 38.9.
 const long MIN_PAIRS = 16384;
 
-int use_pairs(const Geo& g, double c1, bool* yes, PairFields* f)
+// The packed fields of lattice g; false when it cannot be packed, is too small, or the device has no room for
+// them (the scalar form then runs as it did without).
+bool pair_fields(const Geo& g, PairFields* f)
+{
+  if (!qgb::pair_geo(g, &f->pg) || f->pg.pairs < MIN_PAIRS) return false;
+  void** slots[3] = {&f->u, &f->t, &f->p};
+  for (int i = 0; i < 3; ++i)
+    if (get_scratch(f->pg.bytes, 71 + i, slots[i]) != QGB_OK) {
+      (void)cudaGetLastError();
+      for (int j = 0; j < i; ++j) {  // no recorded graph can hold a part of the set
+        cudaFree(*slots[j]);
+        g_ctx.scratch.erase(std::make_pair(f->pg.bytes, 71 + j));
+      }
+      return false;
+    }
+  return true;
+}
+
+bool use_pairs(const Geo& g, double c1, PairFields* f)
 {
   int bs, minb, split, map;
-  *yes = c1 != 0.0 && qgb::force_variant_info_c(g_force_variant[1][1], &bs, &minb, &split, &map) && map == 6 &&
-         qgb::pair_geo(g, &f->pg) && f->pg.pairs >= MIN_PAIRS;
-  if (!*yes) return QGB_OK;
-  QGB_RC(get_scratch(f->pg.bytes, 71, &f->u));
-  QGB_RC(get_scratch(f->pg.bytes, 72, &f->t));
-  return get_scratch(f->pg.bytes, 73, &f->p);
+  return c1 != 0.0 && qgb::force_variant_info_c(g_force_variant[1][1], &bs, &minb, &split, &map) && map == 6 &&
+         pair_fields(g, f);
 }
 
 int pair_pack(const Geo& g, const PairFields& f, const void* natural, void* packed)
@@ -626,7 +640,8 @@ int run_graphed(std::vector<uint64_t> key, F&& body)
 template <typename R>
 int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, double c1, int n_step, double md_time,
                   int integrator, int unit_each, int reunit_every, qgb_halo_hook hook = nullptr,
-                  qgb_field* hook_gf = nullptr, void* hook_user = nullptr, bool hook_shifted = false)
+                  qgb_field* hook_gf = nullptr, void* hook_user = nullptr, bool hook_shifted = false,
+                  const PairFields* pairs = nullptr)
 {
   const double dt = md_time / n_step;
   qgb_field_s shifted;  // tmp, described as a field of gf's shape for the hook
@@ -646,25 +661,22 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
   // force-gradient step, so gf is never read at other links; for leapfrog U is
   // gf itself, so leapfrog keeps the separate evolve).  ev_unit 2 is the
   // re-unitarisation with FP64 arithmetic due after that step.
-  // FP32 with rectangles: after the first link update the fields u, p, t go on in pairs of sites
-  bool pairs = false;
-  PairFields pf;
+  // with `pairs` (FP32, no hook) the fields u, p, t go on in pairs of sites after the first link update
   void *u = gf, *p = gm, *t = tmp;
-  if (sizeof(R) == 4 && !hook) QGB_RC(use_pairs(g, c1, &pairs, &pf));
   auto to_pairs = [&]() -> int {
     if (!pairs) return QGB_OK;
-    u = pf.u;
-    p = pf.p;
-    t = pf.t;
-    QGB_RC(pair_pack(g, pf, gf, u));
-    return pair_pack(g, pf, gm, p);
+    u = pairs->u;
+    p = pairs->p;
+    t = pairs->t;
+    QGB_RC(pair_pack(g, *pairs, gf, u));
+    return pair_pack(g, *pairs, gm, p);
   };
   auto from_pairs = [&](const void* links) -> int {
-    QGB_RC(pair_unpack(g, pf, links, gf));
-    return pair_unpack(g, pf, p, gm);
+    QGB_RC(pair_unpack(g, *pairs, links, gf));
+    return pair_unpack(g, *pairs, p, gm);
   };
   auto launch = [&](qgb::ForceMode mode, const ForceArgs& a) -> int {
-    return pairs ? force_pair(pf, mode, a) : force<R>(g, mode, a);
+    return pairs ? force_pair(*pairs, mode, a) : force<R>(g, mode, a);
   };
   auto update_evolve = [&](const void* U, double h, double eps, bool reunit) -> int {
     ForceArgs b = fargs(U, p, beta, c1, h);
@@ -806,10 +818,8 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
 {
   QGB_RC(no_domain(gf, "gradient flow"));
   const Geo g = geo_of(gf);
-  bool pairs = false;
   PairFields pf;
-  if (gf->prec == QGB_F32 && rk3) QGB_RC(use_pairs(g, c1, &pairs, &pf));
-  if (pairs) {
+  if (gf->prec == QGB_F32 && rk3 && use_pairs(g, c1, &pf)) {
     QGB_RC(pair_pack(g, pf, gf->d, pf.u));
     auto stage = [&](const void* in, void* out, double a, double b, const void* zp, void* zo) -> int {
       ForceArgs fa = fargs(in, out, 3.0, c1, eps);
@@ -1933,7 +1943,10 @@ int qgb_run_hmc_evolve(qgb_field* gm, qgb_field* gf, double beta, double c1, int
   void* tmp = nullptr;
   QGB_RC(get_scratch(gf->bytes, 1, &tmp));
   QGB_RC(ensure_partials((size_t)qgb::reduce_blocks(g) * 2));
+  PairFields pf;
+  const bool pairs = gf->prec == QGB_F32 && use_pairs(g, c1, &pf);
   const std::vector<uint64_t> key = {1,
+                                     key_ptr(pairs ? pf.u : nullptr),
                                      key_ptr(gm->d),
                                      key_ptr(gf->d),
                                      key_ptr(tmp),
@@ -1952,7 +1965,8 @@ int qgb_run_hmc_evolve(qgb_field* gm, qgb_field* gf, double beta, double c1, int
     if (gf->prec == QGB_F64)
       QGB_RC(md_trajectory<double>(g, gf->d, gm->d, tmp, beta, c1, n_step, md_time, integrator, 1, 0));
     else
-      QGB_RC(md_trajectory<float>(g, gf->d, gm->d, tmp, beta, c1, n_step, md_time, integrator, 1, 0));
+      QGB_RC(md_trajectory<float>(g, gf->d, gm->d, tmp, beta, c1, n_step, md_time, integrator, 1, 0, nullptr, nullptr,
+                                  nullptr, false, pairs ? &pf : nullptr));
     QGB_RC(qgb_unitarize(gf));
     return hamiltonian_slots(gm, gf, c1, 3);
   }));
@@ -1983,7 +1997,10 @@ int qgb_run_hmc_evolve_mixed(qgb_field* gm, qgb_field* gf, double beta, double c
   const int nb = qgb::reduce_blocks(g);
   QGB_RC(ensure_partials((size_t)nb * 2));
   const int unit_each = reunit_interval > 0 ? 0 : 1;
+  PairFields pf;
+  const bool pairs = use_pairs(g, c1, &pf);
   const std::vector<uint64_t> key = {2,
+                                     key_ptr(pairs ? pf.u : nullptr),
                                      key_ptr(gm->d),
                                      key_ptr(gf->d),
                                      key_ptr(gf32),
@@ -2009,7 +2026,7 @@ int qgb_run_hmc_evolve_mixed(qgb_field* gm, qgb_field* gf, double beta, double c
       QGB_TRY_CUDA(qgb::launch_finalize(g_ctx.partials, c1 != 0.0 ? 2 : 1, nb, g_ctx.results, 1, g_ctx.stream));
     }
     QGB_RC(md_trajectory<float>(g, gf32, gm32, tmp32, beta, c1, n_step, md_time, integrator, unit_each,
-                                reunit_interval));
+                                reunit_interval, nullptr, nullptr, nullptr, false, pairs ? &pf : nullptr));
     // back to FP64: the links unitarised in the same pass, the momenta with H1's
     // kinetic sum
     {
@@ -2376,14 +2393,10 @@ int qgb_autotune_force(const qgb_field* gf, double c1, int32_t reps, int32_t* be
   QGB_TRY_CUDA(cudaMemcpyAsync(T2, gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   // the shape that runs in pairs of sites is timed on packed copies
   PairFields pf;
-  bool pairs = false;
-  if (gf->prec == QGB_F32 && c1 != 0.0 && qgb::pair_geo(g, &pf.pg) && pf.pg.pairs >= MIN_PAIRS) {
-    QGB_RC(get_scratch(pf.pg.bytes, 71, &pf.u));
-    QGB_RC(get_scratch(pf.pg.bytes, 72, &pf.t));
-    QGB_RC(get_scratch(pf.pg.bytes, 73, &pf.p));
+  const bool pairs = gf->prec == QGB_F32 && c1 != 0.0 && pair_fields(g, &pf);
+  if (pairs) {
     QGB_RC(pair_pack(g, pf, gf->d, pf.u));
     QGB_RC(pair_pack(g, pf, P, pf.p));
-    pairs = true;
   }
   cudaEvent_t e0 = get_event(), e1 = get_event();
   const int nv = qgb::force_variant_count();
