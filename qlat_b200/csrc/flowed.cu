@@ -777,11 +777,17 @@ int flowed_force(qgb_field* gm_force, const qgb_field* gf0, const qgb_field* pre
     a.old = old_of(i);
     FL_RC(launch_flow_step<FLOW_FORWARD>(c, a, steps[i].flow_size));
   }
+  // The steps alternate between the caller's force and F2 so that the last one writes the caller's: F2 holds
+  // words of earlier calls in its padding, and a field's padding is zero.
   void* F = qgb::field_data(gm_force);
-  if (pre) FL_RC(qgb_field_copy(gm_force, pre));
-  else FL_RC(qgb::force_on(c.g, G.p, F, beta, c1));  // the action's force on the flowed field (hmc.cpp:466-490)
+  void *in = n % 2 == 0 ? F : F2.p, *out = n % 2 == 0 ? F2.p : F;
+  if (pre) {
+    FL_RC(qgb_field_copy(gm_force, pre));
+    if (in != F) FL_CUDA(cudaMemcpyAsync(in, F, c.bytes, cudaMemcpyDeviceToDevice, c.st));
+  } else {
+    FL_RC(qgb::force_on(c.g, G.p, in, beta, c1));  // the action's force on the flowed field (hmc.cpp:466-490)
+  }
   // back through the steps (set_gm_force_propagated_det_from_flow, flowed-hmc.cpp:1456-1477)
-  void *in = F, *out = F2.p;
   for (int i = n - 1; i >= 0; --i) {
     FlowArgs a = flow_args(c, G.p, steps[i]);
     a.old = old_of(i);
@@ -798,7 +804,6 @@ int flowed_force(qgb_field* gm_force, const qgb_field* gf0, const qgb_field* pre
     FL_CUDA(cudaGetLastError());
     std::swap(in, out);
   }
-  if (in != F) FL_CUDA(cudaMemcpyAsync(F, in, c.bytes, cudaMemcpyDeviceToDevice, c.st));
   return QGB_OK;
 }
 }  // namespace

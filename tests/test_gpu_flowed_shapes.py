@@ -122,3 +122,28 @@ def test_flow_ln_det_and_force_against_numpy(q, ts, size):
     q.set_gm_force_flowed_no_det(F2, pre, gf, fi)
     q.set_gm_force_flowed(F, gf, ga, fi, with_det=False)
     assert np.linalg.norm(np.asarray(F) - np.asarray(F2)) < 1e-14 * np.linalg.norm(np.asarray(F))
+
+
+# 2 x 6 x 2 x 2 = 48 sites, 6^4 = 1296, 10^4 = 10000: the last block of 32 is half filled
+@pytest.mark.gpu
+@pytest.mark.parametrize("ts", [(2, 6, 2, 2), (6, 6, 6, 6), (10, 10, 10, 10)])
+@pytest.mark.parametrize("n", [0, 1, 2, 5])
+def test_force_leaves_no_words_beyond_its_sites(q, ts, n):
+    """qnorm sums the stored field, padding sites included: it is the image's norm for every number of steps,
+    whatever earlier calls left in the work buffers."""
+    full = q.FlowInfo(q.FlowStepInfo(1 + i % 2, i % 4, 0.1, 1) for i in range(4))
+    big = q.GaugeField(q.Geometry((8, 8, 8, 16)))
+    big.set_rand(q.RngState("flowed-padding"), 0.5, 1)
+    ga = q.GaugeAction(5.5, 0.0)
+    q.set_gm_force_flowed(q.GaugeMomentum(big.geo), big, ga, full)
+    fi = q.FlowInfo(q.FlowStepInfo(1 + i % 2, i % 4, 0.1, 1) for i in range(n))
+    gf = q.GaugeField(q.Geometry(ts))
+    gf.set_rand(q.RngState("flowed-padding"), 0.3, 1)
+    pre, F, F2 = (q.GaugeMomentum(gf.geo) for _ in range(3))
+    q.set_gm_force_flowed(F, gf, ga, fi, with_det=False)
+    q.set_gm_force(pre, q.gf_flow(gf, fi), ga)
+    q.set_gm_force_flowed_no_det(F2, pre, gf, fi)
+    for f in (F, F2):
+        image = float((np.abs(np.asarray(f)) ** 2).sum())
+        assert abs(f.qnorm() - image) < 1e-12 * image  # two orders of one sum of positive terms
+    assert np.linalg.norm(np.asarray(F) - np.asarray(F2)) < 1e-14 * np.linalg.norm(np.asarray(F))
