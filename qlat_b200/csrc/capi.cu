@@ -14,6 +14,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -82,6 +83,7 @@ struct Ctx {
   double* staging = nullptr;
   size_t staging_cap = 0;  // bytes
   std::map<std::pair<size_t, int>, std::vector<void*>> scratch;  // (bytes, tag) -> buffers
+  std::map<std::tuple<size_t, int, int>, void*> adjoint;  // (bytes, AdjField, index) -> the flow adjoint's fields
   bool prof_on = false;
   std::map<std::string, ProfEntry> prof;
   std::vector<cudaEvent_t> event_pool;
@@ -267,20 +269,33 @@ int get_scratch(size_t bytes, int tag, void** out)
   return QGB_OK;
 }
 
-// the flow adjoint's checkpoints and stage fields (no recorded graph uses them)
-void release_adjoint_scratch(int64_t* released)
+// The flow adjoint's fields: the states at the checkpoints, the links before each
+// step of a segment, and the stage fields of those steps (5 j + k: the links
+// after stages 1 and 2 and the three stages' Z).
+enum AdjField { ADJ_CHECKPOINT, ADJ_LINKS, ADJ_STAGE };
+
+int adj_field(size_t bytes, AdjField what, int index, void** out)
 {
-  for (auto it = g_ctx.scratch.begin(); it != g_ctx.scratch.end();) {
-    if (it->first.second < 100 || it->first.second >= 0x7A000) {  // (the other units' tags start there)
-      ++it;
-      continue;
-    }
-    for (void* p : it->second) {
-      cudaFree(p);
-      if (released) *released += (int64_t)it->first.first;
-    }
-    it = g_ctx.scratch.erase(it);
+  void*& p = g_ctx.adjoint[std::make_tuple(bytes, (int)what, index)];
+  if (!p) {
+    const cudaError_t e = cudaMalloc(&p, bytes);
+    if (e != cudaSuccess) p = nullptr;
+    QGB_TRY_CUDA(e);
+    QGB_TRY_CUDA(cudaMemsetAsync(p, 0, bytes, g_ctx.stream));  // the padding sites stay zero, as in get_scratch
   }
+  *out = p;
+  return QGB_OK;
+}
+
+// no recorded graph uses them
+void release_adjoint_fields(int64_t* released)
+{
+  for (auto& kv : g_ctx.adjoint) {
+    if (!kv.second) continue;
+    cudaFree(kv.second);
+    if (released) *released += (int64_t)std::get<0>(kv.first);
+  }
+  g_ctx.adjoint.clear();
 }
 
 void release_field_pool()
@@ -863,12 +878,6 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
 
 // ---- flow adjoint ------------------------------------------------------------
 
-// Scratch of the adjoint: the states at the checkpoints (100 + c), the links
-// before each step of a segment (1000 + j) and its stage fields (2000 + 5 j + k:
-// the links after stages 1 and 2, the three stages' Z).  qgb_field_pool_release
-// gives it back.
-const int ADJ_CHECKPOINT = 100, ADJ_LINKS = 1000, ADJ_STAGES = 100000;
-
 // Stage fields kept between a flow's forward pass and its pull-back: at most this much (40 steps at 16^4 in FP64
 // are 7.0 GiB; keeping them saves the second forward pass, 31.5 -> 24.5 ms a gradient).
 const size_t ADJ_KEEP = (size_t)8 << 30;
@@ -878,15 +887,15 @@ const size_t ADJ_KEEP = (size_t)8 << 30;
 static bool adj_keep_all(size_t bytes, int steps)
 {
   if (steps < 1 || (size_t)5 * steps * bytes > ADJ_KEEP) return false;
-  auto have = [&](int tag) {
-    auto it = g_ctx.scratch.find(std::make_pair(bytes, tag));
-    return it != g_ctx.scratch.end() && !it->second.empty();
+  auto have = [&](AdjField what, int i) {
+    auto it = g_ctx.adjoint.find(std::make_tuple(bytes, (int)what, i));
+    return it != g_ctx.adjoint.end() && it->second;
   };
   size_t need = 0;
   for (int j = 0; j < steps; ++j) {
-    if (!have(ADJ_LINKS + j)) need += bytes;
+    if (!have(ADJ_LINKS, j)) need += bytes;
     for (int k = 0; k < 5; ++k)
-      if (!have(ADJ_STAGES + 5 * j + k)) need += bytes;
+      if (!have(ADJ_STAGE, 5 * j + k)) need += bytes;
   }
   if (need == 0) return true;
   size_t free_bytes = 0, total = 0;
@@ -921,8 +930,8 @@ static int flow_kept(const qgb_field* gf, double eps, double c1, int steps, void
 {
   const Geo g = geo_of(gf);
   std::vector<void*> w(steps + 1), k((size_t)5 * steps);
-  for (int j = 0; j < steps; ++j) QGB_RC(get_scratch(gf->bytes, ADJ_LINKS + j, &w[j]));
-  for (int j = 0; j < 5 * steps; ++j) QGB_RC(get_scratch(gf->bytes, ADJ_STAGES + j, &k[j]));
+  for (int j = 0; j < steps; ++j) QGB_RC(adj_field(gf->bytes, ADJ_LINKS, j, &w[j]));
+  for (int j = 0; j < 5 * steps; ++j) QGB_RC(adj_field(gf->bytes, ADJ_STAGE, j, &k[j]));
   w[steps] = out;
   QGB_TRY_CUDA(cudaMemcpyAsync(w[0], gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   for (int j = 0; j < steps; ++j) QGB_RC(flow_step_kept<R>(g, eps, c1, w[j], w[j + 1], &k[(size_t)5 * j]));
@@ -948,8 +957,8 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
   if (keep_all) every = steps;
   const int ncp = keep_all ? 0 : (steps + every - 1) / every;
   std::vector<void*> cps(ncp), wst(every);
-  for (int i = 0; i < ncp; ++i) QGB_RC(get_scratch(bytes, ADJ_CHECKPOINT + i, &cps[i]));
-  for (int i = 0; i < every; ++i) QGB_RC(get_scratch(bytes, ADJ_LINKS + i, &wst[i]));
+  for (int i = 0; i < ncp; ++i) QGB_RC(adj_field(bytes, ADJ_CHECKPOINT, i, &cps[i]));
+  for (int i = 0; i < every; ++i) QGB_RC(adj_field(bytes, ADJ_LINKS, i, &wst[i]));
   void *W1, *W2, *Wx, *Z0, *Z1, *Z2, *lam, *laml, *mua, *mub;
   QGB_RC(get_scratch(bytes, 41, &W1));
   QGB_RC(get_scratch(bytes, 42, &W2));
@@ -970,11 +979,11 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
   std::vector<void*> kept;
   if (keep) {
     kept.resize((size_t)5 * every);
-    for (int i = 0; i < 5 * every; ++i) QGB_RC(get_scratch(bytes, ADJ_STAGES + i, &kept[i]));
+    for (int i = 0; i < 5 * every; ++i) QGB_RC(adj_field(bytes, ADJ_STAGE, i, &kept[i]));
   }
   // forward pass: checkpoints (the states after 0, every, 2 every, ... steps
-  // in the scratch buffers ADJ_CHECKPOINT + c), unless the caller's forward
-  // flow already left them there
+  // in the checkpoint fields), unless the caller's forward flow already left
+  // them there
   if (keep_all && kept_by_flow == FLOW_KEPT_NONE) QGB_RC(flow_kept<R>(gf, eps, c1, steps, Wx));
   const bool cps_ready = keep_all || kept_by_flow == FLOW_KEPT_CHECKPOINTS;
   if (!cps_ready) QGB_TRY_CUDA(cudaMemcpyAsync(cps[0], gf->d, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
@@ -1203,7 +1212,7 @@ int qgb_field_create(qgb_field** out, const int32_t total_site[4], int32_t multi
       cudaGetLastError();
       cudaStreamSynchronize(g_ctx.stream);
       release_field_pool();
-      release_adjoint_scratch(nullptr);
+      release_adjoint_fields(nullptr);
       e = cudaMalloc(&f->d, f->bytes);
     }
   }
@@ -1244,7 +1253,7 @@ int qgb_field_pool_release(int64_t* released)
   if (released) *released = (int64_t)g_ctx.field_pool_bytes;
   if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
   release_field_pool();
-  release_adjoint_scratch(released);
+  release_adjoint_fields(released);
   return QGB_OK;
 }
 
@@ -2247,7 +2256,7 @@ int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, 
   for (int i = 0; i < steps && !stages; ++i) {
     if (i % every == 0) {
       void* cp = nullptr;
-      QGB_RC(get_scratch(gf->bytes, ADJ_CHECKPOINT + i / every, &cp));
+      QGB_RC(adj_field(gf->bytes, ADJ_CHECKPOINT, i / every, &cp));
       QGB_TRY_CUDA(cudaMemcpyAsync(cp, fv.d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     }
     QGB_RC(flow_step(&fv, epsilon, c1, true));

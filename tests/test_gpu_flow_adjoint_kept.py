@@ -57,3 +57,18 @@ def test_kept_fields_are_given_back(q):
     a, b = np.asarray(long[1]), np.asarray(short[1])
     assert np.linalg.norm(a - b) < 1e-6 * np.linalg.norm(b)
     q.release_field_pool()
+
+
+@pytest.mark.gpu
+def test_many_checkpoints_have_buffers_of_their_own(q):
+    """A flow of 1900 steps (26 GB of links and stage fields of 8^4, not kept) with 950 checkpoints, and with 30:
+    the same launches on the same links, so the same bits."""
+    gf = q.GaugeField(q.Geometry((8, 8, 8, 8)))
+    gf.set_rand(q.RngState("adjoint-kept"), 0.3, 1)
+    few = q.gf_flow_action_grad(gf, 1e-4, 1900, 5.5, checkpoint_every=64)
+    many = q.gf_flow_action_grad(gf, 1e-4, 1900, 5.5, checkpoint_every=2)
+    assert many[0] == few[0] and np.array_equal(np.asarray(many[1]), np.asarray(few[1]))
+    lam = np_field(q, gf, gf)
+    few, many = (q.gf_wilson_flow_vjp(gf, 1e-4, 1900, lam, checkpoint_every=e) for e in (64, 2))
+    assert np.array_equal(np.asarray(many), np.asarray(few))
+    q.release_field_pool()
