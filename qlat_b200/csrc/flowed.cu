@@ -120,7 +120,8 @@ __device__ __forceinline__ M3<double> path_staple(const CField<double>& U, const
 // What k_flow_step does with the masked links after forming their staples C.
 enum FlowMode {
   FLOW_FORWARD = 0,   // U <- exp(-eps TA(U C^+)) U (flowed-hmc.cpp:424-454), the old links kept in `old`
-  FLOW_INVERSE = 1,   // the inverse, by fixed-point iterations (flowed-hmc.cpp:456-490)
+  FLOW_INVERSE = 1,   // the inverse, by fixed-point iterations (flowed-hmc.cpp:456-490); with `old` the staples
+                      // go there and U stays (k_flow_invert)
   FLOW_LN_DET = 2,    // FLOW_FORWARD, and ln det M' of each link
   FLOW_PULL = 3,      // U <- old, then the link's part of the force's pull-back
   FLOW_PULL_DET = 4   // the same with the force of the log-determinant
@@ -129,7 +130,7 @@ enum FlowMode {
 struct FlowArgs {
   Geo g;
   Cx<double>* U;
-  Cx<double>* old;  // the masked links of each site block, i fastest: old[(i / 32 * 9 + k) * 32 + i % 32]
+  Cx<double>* old;  // a matrix per masked link, i fastest: old[(i / 32 * 9 + k) * 32 + i % 32]
   int mask, mu;
   double eps;
   long n;  // masked links
@@ -140,7 +141,38 @@ struct FlowArgs {
   Cx<double>* Y;          // FLOW_PULL*: Z U of each masked link (k_flow_force_step), multiplicity 1
 };
 
-constexpr int FLOW_BS = 256, FLOW_LINKS = FLOW_BS / 8;
+// matrix i of FlowArgs::old
+__device__ __forceinline__ M3<double> ld_link(const Cx<double>* old, long i)
+{
+  const Cx<double>* q = old + ((i >> 5) * 9) * 32 + (i & 31);
+  M3<double> m;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m.e[k] = q[32 * k];
+  return m;
+}
+__device__ __forceinline__ void st_link(Cx<double>* old, long i, const M3<double>& m)
+{
+  Cx<double>* q = old + ((i >> 5) * 9) * 32 + (i & 31);
+#pragma unroll
+  for (int k = 0; k < 9; ++k) q[32 * k] = m.e[k];
+}
+
+// unitarize(exp(e TA(u c^+))) v, and the solution u of u = unitarize(exp(e TA(u c^+))) u1 by n_iter iterations
+__device__ __forceinline__ M3<double> moved_link(const M3<double>& u, const M3<double>& v, const M3<double>& c, double e)
+{
+  M3<double> ex = exp_su3(scale(e, traceless_antiherm(mul_adj(u, c))));
+  unitarize(ex);
+  return mul(ex, v);
+}
+__device__ __forceinline__ M3<double> inverse_link(const M3<double>& u1, const M3<double>& c, double e, int n_iter)
+{
+  M3<double> u0 = u1;
+#pragma unroll 1
+  for (int it = 0; it < n_iter; ++it) u0 = moved_link(u0, u1, c, e);
+  return u0;
+}
+
+constexpr int FLOW_BS = 256, FLOW_LINKS = FLOW_BS / 8, INV_BS = 32;
 constexpr int PAD = 66;  // doubles between two links' 8 x 8 matrices: the four links of a warp in distinct banks
 
 // y = A v for the 8 x 8 matrix at `a` (column-major)
@@ -275,9 +307,7 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
   sum8(c);
   M3<double> u;
   if (PULL) {
-    const Cx<double>* q = a.old + ((i >> 5) * 9) * 32 + (i & 31);
-#pragma unroll
-    for (int k = 0; k < 9; ++k) u.e[k] = q[32 * k];
+    u = ld_link(a.old, i);
     if (b == 0 && i0 < a.n) Uw.st(s, mu, u);  // nobody's staple of this step reads it
   } else {
     u = Uw.ld(s, mu);
@@ -418,22 +448,26 @@ __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
     M3<double> cj;
 #pragma unroll
     for (int k = 0; k < 9; ++k) cj.e[k] = sC[k][threadIdx.x];
+    if (MODE == FLOW_INVERSE && a.old != nullptr) {
+      st_link(a.old, j, cj);
+      return;
+    }
     const M3<double> u1 = Uw.ld(sj, mu);
-    if (a.old != nullptr) {
-      Cx<double>* q = a.old + ((j >> 5) * 9) * 32 + (j & 31);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) q[32 * k] = u1.e[k];
-    }
-    M3<double> u0 = u1;
-    const double e = MODE == FLOW_INVERSE ? a.eps : -a.eps;
-#pragma unroll 1
-    for (int it = 0; it < (MODE == FLOW_INVERSE ? a.n_iter : 1); ++it) {
-      M3<double> ex = exp_su3(scale(e, traceless_antiherm(mul_adj(u0, cj))));
-      unitarize(ex);
-      u0 = mul(ex, u1);
-    }
-    Uw.st(sj, mu, u0);
+    if (a.old != nullptr) st_link(a.old, j, u1);
+    Uw.st(sj, mu, MODE == FLOW_INVERSE ? inverse_link(u1, cj, a.eps, a.n_iter) : moved_link(u1, u1, cj, -a.eps));
   }
+}
+
+// The inverse of a step from the staples in a.old: one thread per masked link, in a launch of its own
+// (qgb_gf_flow_inv).
+template <int SZ>
+__global__ void __launch_bounds__(INV_BS) k_flow_invert(FlowArgs a)
+{
+  const long j = (long)blockIdx.x * INV_BS + threadIdx.x;
+  if (j >= a.n) return;
+  const long s = site_rt(a.g, masked_site<SZ>(a.g, j, a.mask), 0, 0, 1, 0);
+  const WField<double> Uw{a.U, a.g.V};
+  Uw.st(s, a.mu, inverse_link(Uw.ld(s, a.mu), ld_link(a.old, j), a.eps, a.n_iter));
 }
 
 // The part of the force's pull-back that reaches the link (y, nu) through a staple (flowed-hmc.cpp:596-777,
@@ -693,8 +727,25 @@ int qgb_gf_flow_inv(qgb_field* gf, const qgb_field* gf1, const qgb_flow_step* st
   FL_RC(check_output(gf));
   FL_RC(qgb_field_copy(gf, gf1));
   void* U = qgb::field_data(gf);
-  for (int i = n - 1; i >= 0; --i)
-    FL_RC(launch_flow_step<FLOW_INVERSE>(c, flow_args(c, U, steps[i]), steps[i].flow_size));
+  // 50 exponentials a link.  In the tail of k_flow_step they are one warp's work of a block's eight, which holds as
+  // long as no SM has a second block (8 steps of 4096 links: 0.84 ms, and 0.94 with a launch of their own); beyond
+  // that they go one thread per link in warps of their own (6144 links: 0.91 ms against 1.61, 16^4: 1.46 against
+  // 5.52).
+  int dev = 0, sms = 0;
+  FL_CUDA(cudaGetDevice(&dev));
+  FL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  WorkBuf C;
+  if (c.links > (long)FLOW_LINKS * sms) FL_CUDA(C.alloc(c.old_bytes, c.st));
+  for (int i = n - 1; i >= 0; --i) {
+    FlowArgs a = flow_args(c, U, steps[i]);
+    a.old = (Cx<double>*)C.p;
+    FL_RC(launch_flow_step<FLOW_INVERSE>(c, a, steps[i].flow_size));
+    if (C.p == nullptr) continue;
+    const unsigned grid = (unsigned)((c.links + INV_BS - 1) / INV_BS);
+    if (steps[i].flow_size == 1) k_flow_invert<1><<<grid, INV_BS, 0, c.st>>>(a);
+    else k_flow_invert<2><<<grid, INV_BS, 0, c.st>>>(a);
+    FL_CUDA(cudaGetLastError());
+  }
   return QGB_OK;
 }
 

@@ -147,3 +147,30 @@ def test_force_leaves_no_words_beyond_its_sites(q, ts, n):
         image = float((np.abs(np.asarray(f)) ** 2).sum())
         assert abs(f.qnorm() - image) < 1e-12 * image  # two orders of one sum of positive terms
     assert np.linalg.norm(np.asarray(F) - np.asarray(F2)) < 1e-14 * np.linalg.norm(np.asarray(F))
+
+
+@pytest.mark.gpu
+def test_inverse_flow_at_many_links(q):
+    """The inverse on more links than a block per SM holds (16^4: 32768 a step, and 12 x 10 x 10 x 14: 8400, no
+    multiple of 32): the iterations run on all of the GPU.  2048 links are 64 warps of one chain of iterations
+    each; 16 times as many, 7 warps an SM, take 1.7 times as long (with one warp of a block at work and seven waiting,
+    6.6 times)."""
+    import time
+    fi = q.FlowInfo(q.FlowStepInfo(1 + i % 2, i % 4, 0.1, 1) for i in range(8))
+    t = []
+    for ts in [(8, 8, 8, 8), (12, 10, 10, 14), (16, 16, 16, 16)]:
+        gf = q.GaugeField(q.Geometry(ts))
+        gf.set_rand(q.RngState("inverse"), 0.3, 1)
+        out = q.gf_flow(gf, fi)
+        back = q.gf_flow_inv(out, fi)
+        a, b = np.asarray(gf), np.asarray(back)
+        assert np.linalg.norm(a - b) < 1e-12 * np.linalg.norm(a)
+        best = 1e9
+        for _ in range(5):
+            q.synchronize()
+            t0 = time.perf_counter()
+            q.gf_flow_inv(back, out, fi)
+            q.synchronize()
+            best = min(best, time.perf_counter() - t0)
+        t.append(best)
+    assert t[2] < 4 * t[0], t
