@@ -72,6 +72,7 @@ struct ProfEntry {
 struct Ctx {
   bool ready = false;
   int device = 0;
+  int sms = 0;  // multiprocessors
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   double* partials = nullptr;
@@ -131,6 +132,7 @@ int ensure_ctx()
   int n = 0;
   if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) return fail(QGB_ERR_NO_DEVICE, "no CUDA device available");
   QGB_TRY_CUDA(cudaGetDevice(&g_ctx.device));
+  QGB_TRY_CUDA(cudaDeviceGetAttribute(&g_ctx.sms, cudaDevAttrMultiProcessorCount, g_ctx.device));
   QGB_TRY_CUDA(cudaStreamCreateWithFlags(&g_ctx.stream, cudaStreamNonBlocking));
   g_ctx.own_stream = true;
   QGB_TRY_CUDA(cudaMalloc(&g_ctx.results, Ctx::NSLOT * sizeof(double)));
@@ -485,12 +487,7 @@ struct PairFields {
   void *u = nullptr, *t = nullptr, *p = nullptr;  // links, a second link buffer, momenta (or Z)
 };
 
-// Whether the rectangle force of an FP32 run on lattice g goes in pairs: selected (site map 6) and possible, and
-// enough pairs to fill the GPU.  Half as many threads run twice as long, and the fields are packed before and
-// after: 8 force-gradient steps of Iwasaki at 8^4 take 0.61 ms in pairs against 0.52, at 12870 pairs (404 blocks
-// on 148 SMs of 2) 1.36 against 1.39 and the leapfrog 0.436 against 0.425, at 16^4 (32768 pairs) 2.77 against 3.00,
-// at 24^3 x 64 35.0 against 38.9.
-const long MIN_PAIRS = 16384;
+const long MIN_PAIRS = 16384;  // below, half as many threads leave the GPU idle: 8^4, 0.61 ms in pairs against 0.52
 
 // The packed fields of lattice g; false when it cannot be packed, is too small, or the device has no room for
 // them (the scalar form then runs as it did without).
@@ -510,12 +507,46 @@ bool pair_fields(const Geo& g, PairFields* f)
   return true;
 }
 
-bool use_pairs(const Geo& g, double c1, PairFields* f)
+// Time of `blocks` equal blocks at `per` to an SM, in full waves; a last wave of no more than one (two) to an SM takes
+// tail[0] (tail[1]).
+double wave_time(long blocks, int per, const double* tail)
+{
+  const long full = blocks / (per * (long)g_ctx.sms), left = blocks - full * per * g_ctx.sms;
+  return (double)full + (left == 0 ? 0.0 : left <= g_ctx.sms ? tail[0] : left <= 2L * g_ctx.sms ? tail[1] : 1.0);
+}
+
+// Whether a run of `forces` rectangle forces on FP32 links goes in pairs (site map 6), with `passes` fields packed or
+// unpacked around it: if the waves that the force launches save are worth more than the packing, in waves of the
+// scalar form.
+// A wave of pairs does 4/3 of the sites of a scalar one (2 blocks of 128 pairs to an SM against 3 of 128 sites).  What
+// a pair gains on large lattices depends on the paired direction and on its extent: the border copies are 4 / half of
+// the links, and lie in runs of whole blocks of 32 sites along t, in shorter ones along z.  Forces at Iwasaki, scalar /
+// paired time in leapfrog and in force-gradient steps (us a launch in brackets):
+//   paired along t, 24^3 x 64 1.10 (1156 / 1052), 1.13; 24^3 x 12 1.06, 1.08; x 8 1.05, 1.06; x 6 1.02, 1.03; x 4 0.99, 1.01
+//   along z, 24^2 x 64 x 25 1.07, 1.09; x 16 1.05, 1.07; x 8 1.00, 1.01; x 4 0.91, 0.91
+// A pass takes 0.06 to 0.09 of a force.  On small lattices the last wave decides: 14^4 (2.04 waves of pairs, 2.71
+// scalar ones) 0.97, 13^3 x 20 (2.32, 3.10) 1.08, 17^3 x 16 (4.16, 5.54) 1.00, 16^4 (3.46, 4.61) 1.09.
+// Over 95 lattices with nine or ten runs each (1 to 8 steps of both integrators, flow steps) the choice is 0.1% slower
+// on average than the better form every time; where it takes pairs, at most 3% (four forces at 32^4).
+bool pairs_pay(const qgb::PairGeo& pg, int forces, int passes)
+{
+  const double gain = pg.p == 3 ? 0.145 - 0.30 / pg.half : 0.11 - 0.35 / pg.half;
+  static const double scalar_tail[2] = {0.35, 0.5}, pair_tail[2] = {0.56, 1.0};
+  const long ns = 4 * ((2 * pg.pairs + 127) / 128), np = 4 * ((pg.pairs + 127) / 128);
+  const double scalar = wave_time(ns, 3, scalar_tail);
+  const double paired = 4.0 / 3.0 / (1.0 + gain) * wave_time(np, 2, pair_tail);
+  return forces * (scalar - paired) > passes * (0.06 + 0.07 / pg.half) * (double)ns / (3.0 * g_ctx.sms);
+}
+
+bool use_pairs(const Geo& g, double c1, int forces, int passes, PairFields* f)
 {
   int bs, minb, split, map;
-  return c1 != 0.0 && qgb::force_variant_info_c(g_force_variant[1][1], &bs, &minb, &split, &map) && map == 6 &&
-         pair_fields(g, f);
+  if (c1 == 0.0 || !qgb::force_variant_info_c(g_force_variant[1][1], &bs, &minb, &split, &map) || map != 6) return false;
+  return qgb::pair_geo(g, &f->pg) && pairs_pay(f->pg, forces, passes) && pair_fields(g, f);
 }
+
+// force launches of md_trajectory
+int md_forces(int integrator, int n_step) { return integrator == QGB_INTEGRATOR_FORCE_GRADIENT ? 4 * n_step : n_step; }
 
 int pair_pack(const Geo& g, const PairFields& f, const void* natural, void* packed)
 {
@@ -834,7 +865,7 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
   QGB_RC(no_domain(gf, "gradient flow"));
   const Geo g = geo_of(gf);
   PairFields pf;
-  if (gf->prec == QGB_F32 && rk3 && use_pairs(g, c1, &pf)) {
+  if (gf->prec == QGB_F32 && rk3 && use_pairs(g, c1, 3, 2, &pf)) {
     QGB_RC(pair_pack(g, pf, gf->d, pf.u));
     auto stage = [&](const void* in, void* out, double a, double b, const void* zp, void* zo) -> int {
       ForceArgs fa = fargs(in, out, 3.0, c1, eps);
@@ -1953,7 +1984,7 @@ int qgb_run_hmc_evolve(qgb_field* gm, qgb_field* gf, double beta, double c1, int
   QGB_RC(get_scratch(gf->bytes, 1, &tmp));
   QGB_RC(ensure_partials((size_t)qgb::reduce_blocks(g) * 2));
   PairFields pf;
-  const bool pairs = gf->prec == QGB_F32 && use_pairs(g, c1, &pf);
+  const bool pairs = gf->prec == QGB_F32 && use_pairs(g, c1, md_forces(integrator, n_step), 4, &pf);
   const std::vector<uint64_t> key = {1,
                                      key_ptr(pairs ? pf.u : nullptr),
                                      key_ptr(gm->d),
@@ -2007,7 +2038,7 @@ int qgb_run_hmc_evolve_mixed(qgb_field* gm, qgb_field* gf, double beta, double c
   QGB_RC(ensure_partials((size_t)nb * 2));
   const int unit_each = reunit_interval > 0 ? 0 : 1;
   PairFields pf;
-  const bool pairs = use_pairs(g, c1, &pf);
+  const bool pairs = use_pairs(g, c1, md_forces(integrator, n_step), 4, &pf);
   const std::vector<uint64_t> key = {2,
                                      key_ptr(pairs ? pf.u : nullptr),
                                      key_ptr(gm->d),

@@ -137,7 +137,7 @@ static const int N_CORNER_FIELDS = 16;
 // FP32 fields packed in pairs of sites half a lattice apart (force_pair.cu).
 struct PairGeo {
   Geo g;       // the packed field: extent half + 4 along p; its box (bl, bn) the pairs themselves
-  int p;       // the paired direction
+  int p;       // the paired direction: 3, or 2
   int half;    // pairs along p
   long pairs;  // pairs of sites
   long stride; // of the site index along p
