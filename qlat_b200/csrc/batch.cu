@@ -107,12 +107,12 @@ int batch_force(qgb_batch_s* b, qgb::ForceMode mode, const qgb::ForceArgs& a)
 }
 
 template <typename R>
-int batch_evolve(qgb_batch_s* b, void* U, const void* P, double eps, int unit)
+int batch_evolve(qgb_batch_s* b, void* U, const void* P, double eps, int unit, void* W = nullptr)
 {
   qgb::Geo g;
   g.d[0] = g.d[1] = g.d[2] = g.d[3] = 1;
   g.V = b->Vtot;
-  QB_KERNEL(b, qgb::launch_evolve<R>(g, U, P, eps, unit, 0, b->stream));
+  QB_KERNEL(b, qgb::launch_evolve<R>(g, U, P, eps, unit, 0, b->stream, W));
   return QGB_OK;
 }
 
@@ -169,9 +169,9 @@ int batch_md(qgb_batch_s* b, void* gf, void* gm, void* tmp, int n_step, double m
                               b->stream));
   } else if (integrator == QGB_INTEGRATOR_LEAPFROG) {
     // FP64 (re-unitarised after every link step): as the single-lattice FP64 leapfrog, one launch per step
-    QB_RC(batch_evolve<R>(b, gf, gm, 0.5 * dt, unit_each));
-    void* cur = gf;
-    void* nxt = tmp;
+    void* cur = n_step % 2 == 0 ? gf : tmp;
+    void* nxt = n_step % 2 == 0 ? tmp : gf;
+    QB_RC(batch_evolve<R>(b, gf, gm, 0.5 * dt, unit_each, cur));
     for (int i = 0; i < n_step; ++i) {
       qgb::ForceArgs u = bargs(cur, gm, dt, 1);
       u.ev = nxt;
@@ -180,9 +180,6 @@ int batch_md(qgb_batch_s* b, void* gf, void* gm, void* tmp, int n_step, double m
       QB_RC(batch_force<R>(b, qgb::FORCE_LEAPFROG, u));
       std::swap(cur, nxt);
     }
-    if (cur != gf)
-      QB_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(b->Vtot) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
-                              b->stream));
   } else {
     return bfail(QGB_ERR_INVALID_ARG, "unknown integrator");
   }

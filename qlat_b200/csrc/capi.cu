@@ -461,10 +461,10 @@ int force(const Geo& g, qgb::ForceMode mode, const ForceArgs& a0)
 }
 
 template <typename R>
-int evolve(const Geo& g, void* U, const void* P, double eps, int unit)
+int evolve(const Geo& g, void* U, const void* P, double eps, int unit, void* W = nullptr)
 {
   Prof p("evolve");
-  QGB_TRY_CUDA(qgb::launch_evolve<R>(g, U, P, eps, unit, 0, g_ctx.stream));
+  QGB_TRY_CUDA(qgb::launch_evolve<R>(g, U, P, eps, unit, 0, g_ctx.stream, W));
   return QGB_OK;
 }
 
@@ -780,10 +780,11 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
     }
   } else if (integrator == QGB_INTEGRATOR_LEAPFROG && sizeof(R) == 8 && !hook && reunit_every == 0 && unit_each) {
     // FP64 leapfrog, one launch per step: the two half steps of the link update between two forces follow the
-    // momentum update in the force's launch, each unitarised, into the other of two link buffers
-    QGB_RC(evolve<R>(g, gf, gm, 0.5 * dt, unit_each));
-    void* cur = gf;
-    void* nxt = tmp;
+    // momentum update in the force's launch, each unitarised, into the other of two link buffers.  With an odd
+    // number of steps the first half step goes over to tmp, so that the last one ends in gf.
+    void* cur = n_step % 2 == 0 ? gf : tmp;
+    void* nxt = n_step % 2 == 0 ? tmp : gf;
+    QGB_RC(evolve<R>(g, gf, gm, 0.5 * dt, unit_each, cur));
     for (int i = 0; i < n_step; ++i) {
       ForceArgs b = fargs(cur, gm, beta, c1, dt);
       b.ev = nxt;
@@ -791,11 +792,6 @@ int md_trajectory(const Geo& g, void* gf, void* gm, void* tmp, double beta, doub
       b.ev_reps = i + 1 < n_step ? 2 : 1;
       QGB_RC(force<R>(g, qgb::FORCE_LEAPFROG, b));
       std::swap(cur, nxt);
-    }
-    if (cur != gf) {
-      Prof p("copy", 0);
-      QGB_TRY_CUDA(cudaMemcpyAsync(gf, cur, (size_t)qgb::padded_sites(g.V) * 72 * sizeof(R), cudaMemcpyDeviceToDevice,
-                                   g_ctx.stream));
     }
   } else if (integrator == QGB_INTEGRATOR_LEAPFROG) {
     for (int i = 0; i < n_step; ++i) {

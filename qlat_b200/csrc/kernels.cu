@@ -76,30 +76,31 @@ void init_constants()
 }
 
 // ------------------------------------------------------------------------
-// gf_evolve: U = unitarize(exp(eps P) U) (hmc.cpp:311-328, matrix-hmc.h:179-188)
+// gf_evolve: W = unitarize(exp(eps P) U) (hmc.cpp:311-328, matrix-hmc.h:179-188); W may be U
 
 template <typename R>
-__global__ void __launch_bounds__(256) k_evolve(Geo g, Cx<R>* U, const Cx<R>* P, double eps, int unit, int taylor)
+__global__ void __launch_bounds__(256) k_evolve(Geo g, Cx<R>* U, Cx<R>* W, const Cx<R>* P, double eps, int unit,
+                                                int taylor)
 {
   const long s = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= g.V) return;
   const int mu = blockIdx.y;
-  const WField<R> Uf{U, g.V};
+  const WField<R> Uf{U, g.V}, Wf{W, g.V};
   const CField<R> Pf{P, g.V};
   const M3<R> a = scale(R(eps), Pf.ld(s, mu));
   const M3<R> e = taylor ? exp_taylor(a, 20) : exp_ch(a);
   M3<R> un = mul(e, Uf.ld(s, mu));
   if (unit) unitarize(un);
-  Uf.st(s, mu, un);
+  Wf.st(s, mu, un);
 }
 
 template <typename R>
 cudaError_t launch_evolve(const Geo& g, void* U, const void* P, double eps, int unitarize, int taylor,
-                          cudaStream_t st)
+                          cudaStream_t st, void* W)
 {
   const int bs = 256;
   dim3 grid((unsigned)((g.V + bs - 1) / bs), 4);
-  k_evolve<R><<<grid, bs, 0, st>>>(g, (Cx<R>*)U, (const Cx<R>*)P, eps, unitarize, taylor);
+  k_evolve<R><<<grid, bs, 0, st>>>(g, (Cx<R>*)U, (Cx<R>*)(W ? W : U), (const Cx<R>*)P, eps, unitarize, taylor);
   return cudaGetLastError();
 }
 
@@ -1098,7 +1099,7 @@ cudaError_t launch_convert(long n, const void* in, void* out, cudaStream_t st)
 // explicit instantiations
 
 #define QGB_INST(R)                                                                                          \
-  template cudaError_t launch_evolve<R>(const Geo&, void*, const void*, double, int, int, cudaStream_t);    \
+  template cudaError_t launch_evolve<R>(const Geo&, void*, const void*, double, int, int, cudaStream_t, void*); \
   template cudaError_t launch_gm_hamilton<R>(const Geo&, const void*, double*, cudaStream_t);              \
   template cudaError_t launch_action<R>(const Geo&, const void*, int, double*, cudaStream_t, void*);       \
   template cudaError_t launch_qnorm<R>(long, const void*, double*, int, cudaStream_t);                    \

@@ -166,10 +166,10 @@ int batch_force_variant_count();
 int force_variant_info_c(int variant, int* bs, int* minb, int* split, int* map);
 
 // U = exp(eps P) U (optionally unitarized; exp by Cayley-Hamilton series or the
-// reference's order-20 Taylor series).
+// reference's order-20 Taylor series); with W into that field instead.
 template <typename R>
 cudaError_t launch_evolve(const Geo& g, void* U, const void* P, double eps, int unitarize, int taylor,
-                          cudaStream_t st);
+                          cudaStream_t st, void* W = nullptr);
 
 // Unitarize all links of a field with multiplicity m; arithmetic in C.
 template <typename R, typename C>

@@ -47,3 +47,22 @@ def test_fused_leapfrog_matches_composition(q, ts, n_step, c1):
     rs = q.RngState("leapfrog")
     got = b.trajectory([rs.split("gm"), rs], n_step)[0]
     assert abs(got - dh2) < 1e-13 * 24 * geo.total_volume + 1e-12 * abs(dh2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_step", [1, 2, 5])
+def test_steps_end_in_the_callers_links(q, n_step):
+    """No copy of the links from a work buffer: that made one step slower than three separate launches."""
+    gf = q.GaugeField(q.Geometry((4, 4, 4, 6)))
+    gf.set_rand(q.RngState("leapfrog").split("gf"), 0.4, 1)
+    gm = q.GaugeMomentum(gf.geo)
+    gm.set_rand(q.RngState("leapfrog").split("gm"), 1.0)
+    q.prof_reset()
+    q.prof_enable(True)
+    try:
+        q.run_hmc_evolve_pure_gauge(gm, gf, q.GaugeAction(2.3, 0.0), None, n_step, integrator="leapfrog")
+        q.synchronize()
+        got = [q.prof_get(k)[1] for k in ("evolve", "force_leapfrog", "copy")]
+    finally:
+        q.prof_enable(False)
+    assert got == [1, n_step, 0]
