@@ -87,6 +87,12 @@ int qgb_field_destroy(qgb_field* f);
  * does this by itself when cudaMalloc runs out of memory); writes the bytes
  * freed when released is not NULL. */
 int qgb_field_pool_release(int64_t* released);
+/* Bounds on the fields that the flow adjoint keeps, six per step, and holds for
+ * its next call: of a whole flow, also over all lattices together (10 GiB; 0:
+ * always checkpoint and recompute), and of one recomputed segment (5 GiB; 0:
+ * recompute each of its steps twice).  Negative: the default.  Frees what is
+ * held. */
+int qgb_set_flow_adjoint_memory(int64_t flow_bytes, int64_t segment_bytes);
 int qgb_field_info(const qgb_field* f, int32_t total_site[4], int32_t* multiplicity, int32_t* kind,
                    int32_t* precision);
 /* Copy a host buffer in the reference memory image into the field (and back).
@@ -244,8 +250,10 @@ int qgb_gf_wilson_flow(qgb_field* gf, double flow_time, int32_t steps, double c1
  * (gf_wilson_flow_step, wilson-flow.cpp:29-50, with the flow force of
  * GaugeAction(3, c1), set_wilson_flow_z at wilson-flow.cpp:12-17: Wilson,
  * Iwasaki, DBW2 or any c1): given the cotangent at the flowed field, writes
- * the cotangent at gf.  Forward states are checkpointed every
- * `checkpoint_every` steps and recomputed. */
+ * the cotangent at gf.  A flow whose links and stage fields fit a bound
+ * (qgb_set_flow_adjoint_memory) and the device keeps them all; otherwise
+ * forward states are checkpointed every `checkpoint_every` steps and
+ * recomputed. */
 int qgb_gf_wilson_flow_vjp(const qgb_field* gf, double epsilon, int32_t steps, double c1, int32_t checkpoint_every,
                            const qgb_field* cotangent, qgb_field* grad);
 /* L = gf_hamilton_node(V_t, GaugeAction(beta, c1_loss)) of the flowed field

@@ -31,7 +31,7 @@ from .slabs import TimeSlabs, run_hmc_evolve_slabs, run_hmc_pure_gauge_slabs
 from .domains import Domains, domain_layout, run_hmc_evolve_domains, run_hmc_pure_gauge_domains
 from .flow_adjoint import (FlowedWilsonAction, gf_flow_action, gf_flow_action_grad, gf_wilson_flow_vjp,
                            run_flowed_hmc_pure_gauge, set_anti_hermitian_matrix_from_basis,
-                           set_basis_from_anti_hermitian_matrix)
+                           set_basis_from_anti_hermitian_matrix, set_flow_adjoint_memory)
 from .wilson_flow import (gf_energy_density_dir_field, topology_charge_5,
                           gf_energy_density, gf_energy_density_field, gf_energy_derivative_density_field,
                           gf_topology, gf_topology_clf, gf_topology_field, gf_topology_field_clf, gf_topology_terms,

@@ -33,6 +33,7 @@ SIGNATURES = {
     "qgb_field_create": [c_field_p, i32x4, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32],
     "qgb_field_destroy": [c_field],
     "qgb_field_pool_release": [c_i64_p],
+    "qgb_set_flow_adjoint_memory": [ctypes.c_int64, ctypes.c_int64],
     "qgb_nersc_write_host": [ctypes.c_char_p, c_dbl_p, i32x4, ctypes.c_double, ctypes.c_double, ctypes.c_char_p,
                              ctypes.c_char_p, ctypes.c_char_p, ctypes.c_char_p, ctypes.c_double, ctypes.c_int64,
                              c_i64_p],

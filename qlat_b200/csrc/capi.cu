@@ -289,15 +289,21 @@ int adj_field(size_t bytes, AdjField what, int index, void** out)
   return QGB_OK;
 }
 
-// no recorded graph uses them
-void release_adjoint_fields(int64_t* released)
+// Frees the adjoint's fields but the first n[what] of each kind with `bytes` bytes (no recorded graph uses them).
+void release_adjoint_fields(int64_t* released, size_t bytes = 0, const int* n = nullptr)
 {
-  for (auto& kv : g_ctx.adjoint) {
-    if (!kv.second) continue;
-    cudaFree(kv.second);
-    if (released) *released += (int64_t)std::get<0>(kv.first);
+  for (auto it = g_ctx.adjoint.begin(); it != g_ctx.adjoint.end();) {
+    const auto& key = it->first;
+    if (n && std::get<0>(key) == bytes && std::get<2>(key) < n[std::get<1>(key)]) {
+      ++it;
+      continue;
+    }
+    if (it->second) {
+      cudaFree(it->second);
+      if (released) *released += (int64_t)std::get<0>(key);
+    }
+    it = g_ctx.adjoint.erase(it);
   }
-  g_ctx.adjoint.clear();
 }
 
 void release_field_pool()
@@ -905,32 +911,90 @@ static int flow_step(qgb_field* gf, double eps, double c1, bool rk3)
 
 // ---- flow adjoint ------------------------------------------------------------
 
-// Stage fields kept between a flow's forward pass and its pull-back: at most this much (40 steps at 16^4 in FP64
-// are 7.0 GiB; keeping them saves the second forward pass, 31.5 -> 24.5 ms a gradient).
-const size_t ADJ_KEEP = (size_t)8 << 30;
+// Bounds on the links and stage fields (six fields a step) that the adjoint keeps: of a whole flow between its
+// forward pass and its pull-back, and of a segment's recomputation (qgb_set_flow_adjoint_memory).  40 steps at 16^4
+// in FP64 are 8.4 GiB; keeping them saves the second forward pass, 31.5 -> 24.5 ms a gradient.
+const size_t ADJ_FLOW_BYTES = (size_t)10 << 30, ADJ_SEGMENT_BYTES = (size_t)5 << 30;
+size_t g_adj_flow_bytes = ADJ_FLOW_BYTES, g_adj_segment_bytes = ADJ_SEGMENT_BYTES;
 
-// Whether every step of the flow can keep its stage fields, so that nothing is recomputed: they fit the bound
-// and the device's free memory (with 2 GiB to spare), or are there already.
-static bool adj_keep_all(size_t bytes, int steps)
+// The buffers of one adjoint call.
+struct AdjPlan {
+  bool all = false;      // every step keeps its links and stage fields: one segment, nothing is recomputed
+  bool segment = false;  // the steps of a segment keep them once it is recomputed
+  int every = 0;         // steps of a segment
+  std::vector<void*> cps, links, stages;  // checkpoints (none with `all`), a segment's links and stage fields
+  void* w[10];                            // work fields
+};
+
+static bool adj_fits(size_t bytes, int steps, size_t bound) { return (size_t)steps <= bound / (6 * bytes); }
+
+// Room for a call that uses n[kind] fields of each kind with `bytes` bytes and leaves the device 2 GiB: frees what it
+// does not use if the adjoint would hold more than its bound otherwise, and that and the field pool if the device
+// lacks the room.  False, with nothing freed, if that would not do.
+static bool adj_room(size_t bytes, const int* n)
 {
-  if (steps < 1 || (size_t)5 * steps * bytes > ADJ_KEEP) return false;
-  auto have = [&](AdjField what, int i) {
-    auto it = g_ctx.adjoint.find(std::make_tuple(bytes, (int)what, i));
-    return it != g_ctx.adjoint.end() && it->second;
-  };
-  size_t need = 0;
-  for (int j = 0; j < steps; ++j) {
-    if (!have(ADJ_LINKS, j)) need += bytes;
-    for (int k = 0; k < 5; ++k)
-      if (!have(ADJ_STAGE, 5 * j + k)) need += bytes;
+  size_t held = 0, own = 0;
+  for (auto& kv : g_ctx.adjoint) {
+    if (!kv.second) continue;
+    held += std::get<0>(kv.first);
+    if (std::get<0>(kv.first) == bytes && std::get<2>(kv.first) < n[std::get<1>(kv.first)]) own += bytes;
   }
+  const size_t need = ((size_t)n[0] + n[1] + n[2]) * bytes - own, want = need + ((size_t)2 << 30);
   if (need == 0) return true;
   size_t free_bytes = 0, total = 0;
   if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess) {
     (void)cudaGetLastError();
     return false;
   }
-  return free_bytes >= need + ((size_t)2 << 30);
+  if (free_bytes + (held - own) + g_ctx.field_pool_bytes < want) return false;
+  if (free_bytes < want) release_field_pool();
+  if (free_bytes < want || held + need > g_adj_flow_bytes) release_adjoint_fields(nullptr, bytes, n);
+  return true;
+}
+
+static int adj_fields(size_t bytes, AdjField what, int n, std::vector<void*>* out)
+{
+  out->resize(n);
+  for (int i = 0; i < n; ++i) QGB_RC(adj_field(bytes, what, i, &(*out)[i]));
+  return QGB_OK;
+}
+
+// The buffers for a flow of `steps` steps with a checkpoint every `every` of them (not used where the whole flow is
+// kept).  What does not fit the bounds or the device is recomputed, which changes at most rounding.
+static int adj_plan(size_t bytes, int steps, int every, AdjPlan* p)
+{
+  for (int i = 0; i < 10; ++i) QGB_RC(get_scratch(bytes, 41 + i, &p->w[i]));
+  if (adj_fits(bytes, steps, g_adj_flow_bytes)) {
+    const int n[3] = {0, steps, 5 * steps};
+    if (adj_room(bytes, n)) {
+      p->every = steps;
+      p->all = p->segment = adj_fields(bytes, ADJ_LINKS, steps, &p->links) == QGB_OK &&
+                            adj_fields(bytes, ADJ_STAGE, 5 * steps, &p->stages) == QGB_OK;
+      if (p->all) return QGB_OK;
+      (void)cudaGetLastError();
+      release_adjoint_fields(nullptr);
+    }
+  }
+  for (int i = 0; i < 2; ++i) {  // flow_step's, before the rest is taken
+    void* t = nullptr;
+    QGB_RC(get_scratch(bytes, 21 + i, &t));
+  }
+  int n[3] = {(steps - 1) / every + 1, every, 0};
+  p->every = every;
+  if (adj_fits(bytes, every, g_adj_segment_bytes)) {
+    n[ADJ_STAGE] = 5 * every;
+    p->segment = adj_room(bytes, n) && adj_fields(bytes, ADJ_STAGE, 5 * every, &p->stages) == QGB_OK;
+    (void)cudaGetLastError();
+  }
+  if (!p->segment) {
+    n[ADJ_STAGE] = 0;
+    if (!adj_room(bytes, n)) {
+      release_field_pool();
+      release_adjoint_fields(nullptr, bytes, n);
+    }
+  }
+  QGB_RC(adj_fields(bytes, ADJ_CHECKPOINT, n[ADJ_CHECKPOINT], &p->cps));
+  return adj_fields(bytes, ADJ_LINKS, every, &p->links);
 }
 
 // One RK3 step in -> out, keeping its stage fields k: the links after stages 1
@@ -951,76 +1015,49 @@ static int flow_step_kept(const Geo& g, double eps, double c1, const void* in, v
   return stage(k[1], out, 0.75, -1.0, k[3], k[4]);
 }
 
-// The flow of gf into `out`, keeping every step's links and stage fields (adj_keep_all).
+// The flow of gf into `out`, keeping every step's links and stage fields (AdjPlan::all).
 template <typename R>
-static int flow_kept(const qgb_field* gf, double eps, double c1, int steps, void* out)
+static int flow_kept(const qgb_field* gf, double eps, double c1, int steps, const AdjPlan& p, void* out)
 {
   const Geo g = geo_of(gf);
-  std::vector<void*> w(steps + 1), k((size_t)5 * steps);
-  for (int j = 0; j < steps; ++j) QGB_RC(adj_field(gf->bytes, ADJ_LINKS, j, &w[j]));
-  for (int j = 0; j < 5 * steps; ++j) QGB_RC(adj_field(gf->bytes, ADJ_STAGE, j, &k[j]));
-  w[steps] = out;
-  QGB_TRY_CUDA(cudaMemcpyAsync(w[0], gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
-  for (int j = 0; j < steps; ++j) QGB_RC(flow_step_kept<R>(g, eps, c1, w[j], w[j + 1], &k[(size_t)5 * j]));
+  QGB_TRY_CUDA(cudaMemcpyAsync(p.links[0], gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+  for (int j = 0; j < steps; ++j)
+    QGB_RC(flow_step_kept<R>(g, eps, c1, p.links[j], j + 1 < steps ? p.links[j + 1] : out, &p.stages[(size_t)5 * j]));
   return QGB_OK;
 }
 
-// What the forward flow has left for the pull-back.
-enum FlowKept { FLOW_KEPT_NONE, FLOW_KEPT_CHECKPOINTS, FLOW_KEPT_STAGES };
-
 // Pull a cotangent back through RK3 flow steps (adjoint.cu): checkpoints every
-// `every` steps, each segment recomputed forward, each step's three stages
+// p.every steps, each segment recomputed forward, each step's three stages
 // recomputed with their Z fields, then pulled back stage by stage.  When every
-// step can keep its stage fields there is one segment, and none of it is
-// recomputed if the caller's forward flow has left them (FLOW_KEPT_STAGES).
+// step keeps its stage fields there is one segment, and none of it is
+// recomputed.  forward_done: the caller's flow has left the checkpoints or the
+// kept fields.
 template <typename R>
-static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, int every, const void* lam_in,
-                         void* grad, FlowKept kept_by_flow = FLOW_KEPT_NONE)
+static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, const AdjPlan& p, const void* lam_in,
+                         void* grad, bool forward_done)
 {
   const Geo g = geo_of(gf);
   const size_t bytes = gf->bytes;
-  const bool keep_all = kept_by_flow == FLOW_KEPT_STAGES ||
-                        (kept_by_flow == FLOW_KEPT_NONE && adj_keep_all(bytes, steps));
-  if (keep_all) every = steps;
-  const int ncp = keep_all ? 0 : (steps + every - 1) / every;
-  std::vector<void*> cps(ncp), wst(every);
-  for (int i = 0; i < ncp; ++i) QGB_RC(adj_field(bytes, ADJ_CHECKPOINT, i, &cps[i]));
-  for (int i = 0; i < every; ++i) QGB_RC(adj_field(bytes, ADJ_LINKS, i, &wst[i]));
-  void *W1, *W2, *Wx, *Z0, *Z1, *Z2, *lam, *laml, *mua, *mub;
-  QGB_RC(get_scratch(bytes, 41, &W1));
-  QGB_RC(get_scratch(bytes, 42, &W2));
-  QGB_RC(get_scratch(bytes, 43, &Wx));
-  QGB_RC(get_scratch(bytes, 44, &Z0));
-  QGB_RC(get_scratch(bytes, 45, &Z1));
-  QGB_RC(get_scratch(bytes, 46, &Z2));
-  QGB_RC(get_scratch(bytes, 47, &lam));
-  QGB_RC(get_scratch(bytes, 48, &laml));
-  QGB_RC(get_scratch(bytes, 49, &mua));
-  QGB_RC(get_scratch(bytes, 50, &mub));
+  const bool keep_all = p.all, keep = p.segment;
+  const int every = p.every, ncp = (int)p.cps.size();
+  const std::vector<void*>&cps = p.cps, &wst = p.links, &kept = p.stages;
+  void *W1 = p.w[0], *W2 = p.w[1], *Wx = p.w[2], *Z0 = p.w[3], *Z1 = p.w[4], *Z2 = p.w[5], *lam = p.w[6],
+       *laml = p.w[7], *mua = p.w[8], *mub = p.w[9];
   void* const one[5] = {W1, W2, Z0, Z1, Z2};
   auto step = [&](const void* in, void* out) -> int { return flow_step_kept<R>(g, eps, c1, in, out, one); };
-  // When the five stage fields of every step of a segment fit in 4 GiB, the
-  // segment's recomputation keeps them, and the pull-back reads them instead
-  // of recomputing each step a second time.
-  const bool keep = keep_all || (size_t)5 * every * bytes <= ((size_t)4 << 30);
-  std::vector<void*> kept;
-  if (keep) {
-    kept.resize((size_t)5 * every);
-    for (int i = 0; i < 5 * every; ++i) QGB_RC(adj_field(bytes, ADJ_STAGE, i, &kept[i]));
-  }
-  // forward pass: checkpoints (the states after 0, every, 2 every, ... steps
-  // in the checkpoint fields), unless the caller's forward flow already left
-  // them there
-  if (keep_all && kept_by_flow == FLOW_KEPT_NONE) QGB_RC(flow_kept<R>(gf, eps, c1, steps, Wx));
-  const bool cps_ready = keep_all || kept_by_flow == FLOW_KEPT_CHECKPOINTS;
-  if (!cps_ready) QGB_TRY_CUDA(cudaMemcpyAsync(cps[0], gf->d, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
-  for (int c = 1; c < ncp && !cps_ready; ++c) {
-    QGB_TRY_CUDA(cudaMemcpyAsync(Wx, cps[c - 1], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
-    for (int j = 0; j < every; ++j) {
-      QGB_RC(step(Wx, wst[0]));
-      QGB_TRY_CUDA(cudaMemcpyAsync(Wx, wst[0], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+  // forward pass: the kept fields, or the checkpoints (the states after 0,
+  // every, 2 every, ... steps)
+  if (!forward_done && keep_all) QGB_RC(flow_kept<R>(gf, eps, c1, steps, p, Wx));
+  if (!forward_done && !keep_all) {
+    QGB_TRY_CUDA(cudaMemcpyAsync(cps[0], gf->d, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+    for (int c = 1; c < ncp; ++c) {
+      QGB_TRY_CUDA(cudaMemcpyAsync(Wx, cps[c - 1], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+      for (int j = 0; j < every; ++j) {
+        QGB_RC(step(Wx, wst[0]));
+        QGB_TRY_CUDA(cudaMemcpyAsync(Wx, wst[0], bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+      }
+      QGB_TRY_CUDA(cudaMemcpyAsync(cps[c], Wx, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     }
-    QGB_TRY_CUDA(cudaMemcpyAsync(cps[c], Wx, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   }
   QGB_TRY_CUDA(cudaMemcpyAsync(lam, lam_in, bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
   // backward pass
@@ -1040,7 +1077,7 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
       // stage fields of this step: wst[j], w1, w2 and z0, z1, z2
       const void *w1 = W1, *w2 = W2, *z0 = Z0, *z1 = Z1, *z2 = Z2;
       if (keep) {
-        void** k = &kept[(size_t)5 * j];
+        void* const* k = &kept[(size_t)5 * j];
         w1 = k[0];
         w2 = k[1];
         z0 = k[2];
@@ -1050,7 +1087,7 @@ static int flow_vjp_impl(const qgb_field* gf, double eps, double c1, int steps, 
         QGB_RC(step(wst[j], Wx));
       }
       {
-        Prof p("flow_adjoint", 6);
+        Prof prof("flow_adjoint", 6);
         // stage 3: W3 = exp(eps Z2) W2, Z2 = 3/4 F(W2) - Z1
         QGB_TRY_CUDA(qgb::launch_flow_adj_local<R>(g.V, lam, z2, nullptr, 0.0, eps, mua, laml, g_ctx.stream));
         QGB_TRY_CUDA(qgb::launch_force_vjp<R>(g, w2, mua, laml, lam, 3.0, c1, 0.75, g_ctx.stream));
@@ -1281,6 +1318,16 @@ int qgb_field_pool_release(int64_t* released)
   if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
   release_field_pool();
   release_adjoint_fields(released);
+  return QGB_OK;
+}
+
+int qgb_set_flow_adjoint_memory(int64_t flow_bytes, int64_t segment_bytes)
+{
+  std::lock_guard<std::recursive_mutex> lock(g_mu);
+  if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
+  release_adjoint_fields(nullptr);
+  g_adj_flow_bytes = flow_bytes < 0 ? ADJ_FLOW_BYTES : (size_t)flow_bytes;
+  g_adj_segment_bytes = segment_bytes < 0 ? ADJ_SEGMENT_BYTES : (size_t)segment_bytes;
   return QGB_OK;
 }
 
@@ -2251,9 +2298,10 @@ int qgb_gf_wilson_flow_vjp(const qgb_field* gf, double epsilon, int32_t steps, d
     QGB_TRY_CUDA(cudaMemcpyAsync(grad->d, cotangent->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     return QGB_OK;
   }
-  const int every = checkpoint_every < steps ? checkpoint_every : steps;
-  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, every, cotangent->d, grad->d);
-  return flow_vjp_impl<float>(gf, epsilon, c1, steps, every, cotangent->d, grad->d);
+  AdjPlan p;
+  QGB_RC(adj_plan(gf->bytes, steps, checkpoint_every < steps ? checkpoint_every : steps, &p));
+  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, p, cotangent->d, grad->d, false);
+  return flow_vjp_impl<float>(gf, epsilon, c1, steps, p, cotangent->d, grad->d, false);
 }
 
 int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, double c1, int32_t checkpoint_every,
@@ -2267,26 +2315,27 @@ int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, 
   QGB_RC(get_scratch(gf->bytes, 61, &V));
   QGB_RC(get_scratch(gf->bytes, 62, &lamN));
   // flowed field V_t, keeping on the way what flow_vjp_impl reads: every step's
-  // links and stage fields if they fit, or the checkpoints (the states after 0,
-  // every, 2 every, ... steps)
-  const bool stages = adj_keep_all(gf->bytes, steps);
-  const int every = steps > 0 ? (checkpoint_every < steps ? checkpoint_every : steps) : 1;
+  // links and stage fields, or the checkpoints (the states after 0, every, 2
+  // every, ... steps).  Every buffer is there before flow_step swaps V with
+  // one of its own.
+  AdjPlan p;
+  if (steps > 0) {
+    QGB_RC(no_domain(gf, "gradient flow"));
+    QGB_RC(adj_plan(gf->bytes, steps, checkpoint_every < steps ? checkpoint_every : steps, &p));
+  }
   qgb_field_s fv = *gf;
   fv.d = V;
-  if (stages) {
-    QGB_RC(no_domain(gf, "gradient flow"));
-    if (gf->prec == QGB_F64) QGB_RC(flow_kept<double>(gf, epsilon, c1, steps, V));
-    else QGB_RC(flow_kept<float>(gf, epsilon, c1, steps, V));
+  if (p.all && gf->prec == QGB_F64) {
+    QGB_RC(flow_kept<double>(gf, epsilon, c1, steps, p, V));
+  } else if (p.all) {
+    QGB_RC(flow_kept<float>(gf, epsilon, c1, steps, p, V));
   } else {
     QGB_TRY_CUDA(cudaMemcpyAsync(V, gf->d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
-  }
-  for (int i = 0; i < steps && !stages; ++i) {
-    if (i % every == 0) {
-      void* cp = nullptr;
-      QGB_RC(adj_field(gf->bytes, ADJ_CHECKPOINT, i / every, &cp));
-      QGB_TRY_CUDA(cudaMemcpyAsync(cp, fv.d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+    for (int i = 0; i < steps; ++i) {
+      if (i % p.every == 0)
+        QGB_TRY_CUDA(cudaMemcpyAsync(p.cps[i / p.every], fv.d, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
+      QGB_RC(flow_step(&fv, epsilon, c1, true));
     }
-    QGB_RC(flow_step(&fv, epsilon, c1, true));
   }
   V = fv.d;  // flow_step hands the result buffer to the handle
   // loss and its gradient at V_t: dL = -2 <F(V_t), X> in the su(3) pairing
@@ -2307,9 +2356,8 @@ int qgb_gf_flow_action_grad(const qgb_field* gf, double epsilon, int32_t steps, 
     QGB_TRY_CUDA(cudaMemcpyAsync(grad->d, lamN, gf->bytes, cudaMemcpyDeviceToDevice, g_ctx.stream));
     return QGB_OK;
   }
-  const FlowKept kept = stages ? FLOW_KEPT_STAGES : FLOW_KEPT_CHECKPOINTS;
-  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, every, lamN, grad->d, kept);
-  return flow_vjp_impl<float>(gf, epsilon, c1, steps, every, lamN, grad->d, kept);
+  if (gf->prec == QGB_F64) return flow_vjp_impl<double>(gf, epsilon, c1, steps, p, lamN, grad->d, true);
+  return flow_vjp_impl<float>(gf, epsilon, c1, steps, p, lamN, grad->d, true);
 }
 
 int qgb_set_anti_hermitian_matrix_from_basis(qgb_field* fc, const qgb_field* basis)

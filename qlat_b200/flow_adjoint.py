@@ -7,7 +7,8 @@ delta_ab).  The gauge action's gradient is then -2 x set_gm_force, because
 Qlattice's momenta have kinetic energy sum_a p_a^2 (hmc.cpp:151-173).
 
 - ``gf_wilson_flow_vjp``: cotangent at the flowed field -> cotangent at the
-  initial field, through RK3 Wilson-flow steps (checkpoints every k steps).
+  initial field, through RK3 Wilson-flow steps (which are kept, or recomputed
+  from checkpoints every k steps: ``set_flow_adjoint_memory``).
 - ``gf_flow_action_grad``: L = gauge action of the flowed field, and dL/dU.
 - ``FlowedWilsonAction``: a torch.autograd.Function of the su(3) coordinates
   omega (shape (V, 4, 8)) of U = exp(omega . T) U0.
@@ -33,6 +34,14 @@ def set_anti_hermitian_matrix_from_basis(fc, basis: FieldRealD):
 def set_basis_from_anti_hermitian_matrix(basis: FieldRealD, fc):
     """basis[x, 8 m + a] = coefficient of T_a in fc[x, m] (hmc.pyx set_basis_from_anti_hermitian_matrix)."""
     call("qgb_set_basis_from_anti_hermitian_matrix", basis.handle, fc.handle)
+
+
+def set_flow_adjoint_memory(flow_bytes: int | None = None, segment_bytes: int | None = None) -> None:
+    """Bounds on the links and stage fields that the flow adjoint keeps, six fields per step, and holds for its next
+    call: of a whole flow, also over all lattices together (default 10 GiB; 0: always checkpoint and recompute), and
+    of one recomputed segment (default 5 GiB; 0: each of its steps is recomputed twice).  Frees what is held."""
+    call("qgb_set_flow_adjoint_memory", -1 if flow_bytes is None else int(flow_bytes),
+         -1 if segment_bytes is None else int(segment_bytes))
 
 
 def gf_wilson_flow_vjp(gf: GaugeField, epsilon: float, steps: int, cotangent, *, c1: float = 0.0,
