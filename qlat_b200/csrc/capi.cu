@@ -55,7 +55,10 @@ int fail(int code, const std::string& msg)
 #define QGB_TRY_CUDA(expr)                                                             \
   do {                                                                                 \
     cudaError_t e_ = (expr);                                                           \
-    if (e_ != cudaSuccess) return fail(QGB_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_)); \
+    if (e_ != cudaSuccess) {                                                           \
+      (void)cudaGetLastError(); /* not the next launch's */                            \
+      return fail(QGB_ERR_CUDA, std::string(#expr) + ": " + cudaGetErrorString(e_));   \
+    }                                                                                  \
   } while (0)
 
 #define QGB_CHECK(cond, code, msg) \
@@ -240,6 +243,7 @@ int ensure_partials(size_t n)
   if (g_ctx.partials_cap >= n) return QGB_OK;
   if (g_ctx.partials) cudaFree(g_ctx.partials);
   g_ctx.partials = nullptr;
+  g_ctx.partials_cap = 0;
   QGB_TRY_CUDA(cudaMalloc(&g_ctx.partials, n * sizeof(double)));
   g_ctx.partials_cap = n;
   return QGB_OK;
@@ -250,6 +254,7 @@ int ensure_staging(size_t bytes)
   if (g_ctx.staging_cap >= bytes) return QGB_OK;
   if (g_ctx.staging) cudaFree(g_ctx.staging);
   g_ctx.staging = nullptr;
+  g_ctx.staging_cap = 0;
   QGB_TRY_CUDA(cudaMalloc(&g_ctx.staging, bytes));
   g_ctx.staging_cap = bytes;
   return QGB_OK;

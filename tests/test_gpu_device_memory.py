@@ -1,0 +1,63 @@
+"""A device that another program has filled: what the library does when an
+allocation of its own fails.  Each case is a process of its own, so that the
+library starts without buffers of earlier tests."""
+
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+PRELUDE = '''
+import numpy as np, torch
+import qlat_b200 as q
+
+def links(ts):
+    gf = q.GaugeField(q.Geometry(ts))
+    gf.set_rand(q.RngState("memory"), 0.3, 1)
+    return gf
+
+class Filled:
+    """All of the device but `spare` bytes in other hands."""
+    def __init__(self, spare):
+        self.spare = spare
+    def __enter__(self):
+        q.synchronize()
+        torch.cuda.empty_cache()
+        self.t = torch.empty(torch.cuda.mem_get_info()[0] - self.spare, dtype=torch.uint8, device="cuda")
+    def __exit__(self, *a):
+        del self.t
+        torch.cuda.empty_cache()
+'''
+
+
+def run(q, code):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code)], cwd=ROOT, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+@pytest.mark.gpu
+def test_transfer_without_room_leaves_the_next_ones_usable(q):
+    """The staging buffer has 2 MB, a transfer of 75 MB cannot enlarge it, and the next needs the 2 MB again."""
+    run(q, '''
+        a, b = links((8, 8, 8, 8)), links((16, 16, 16, 32))
+        small = a.to_numpy()
+        with Filled(32 << 20):
+            for _ in range(2):
+                try:
+                    b.to_numpy()
+                except q.QlatB200Error:
+                    pass
+                else:
+                    raise SystemExit("the transfer found room")
+                assert np.array_equal(a.to_numpy(), small)
+                a.from_numpy(small)
+                assert abs(q.gf_avg_plaq(a)) < 1
+        big = b.to_numpy()
+        b.from_numpy(big)
+        assert np.array_equal(b.to_numpy(), big) and np.array_equal(a.to_numpy(), small)
+    ''')
