@@ -23,6 +23,7 @@
 
 #include "../../include/qlat_b200.h"
 #include "kernels.h"
+#include "work_pool.h"
 
 namespace qgb
 {
@@ -279,7 +280,7 @@ int qgb_batch_create(qgb_batch** out, int32_t n_chains, const int32_t* total_sit
   const size_t b64 = (size_t)qgb::padded_sites(b->Vtot) * 72 * sizeof(double), b32 = b64 / 2;
   cudaError_t e = cudaSuccess;
   auto A = [&](void** p, size_t bytes) {
-    if (e == cudaSuccess) e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) e = qgb::alloc_or_release(p, bytes);
     if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);  // padding sites stay zero
   };
   A((void**)&b->d_offs, (n_chains + 1) * sizeof(long));

@@ -88,6 +88,7 @@ struct Ctx {
   size_t staging_cap = 0;  // bytes
   std::map<std::pair<size_t, int>, std::vector<void*>> scratch;  // (bytes, tag) -> buffers
   std::map<std::tuple<size_t, int, int>, void*> adjoint;  // (bytes, AdjField, index) -> the flow adjoint's fields
+  bool adjoint_busy = false;  // a call is using them
   bool prof_on = false;
   std::map<std::string, ProfEntry> prof;
   std::vector<cudaEvent_t> event_pool;
@@ -238,61 +239,10 @@ long n_reals(const qgb_field_s* f) { return f->V * f->mult * (long)elem_reals(f)
 // elementwise kernels run over all of it, the padding is zero)
 long n_store(const qgb_field_s* f) { return qgb::padded_sites(f->V) * f->mult * (long)elem_reals(f); }
 
-int ensure_partials(size_t n)
-{
-  if (g_ctx.partials_cap >= n) return QGB_OK;
-  if (g_ctx.partials) cudaFree(g_ctx.partials);
-  g_ctx.partials = nullptr;
-  g_ctx.partials_cap = 0;
-  QGB_TRY_CUDA(cudaMalloc(&g_ctx.partials, n * sizeof(double)));
-  g_ctx.partials_cap = n;
-  return QGB_OK;
-}
-
-int ensure_staging(size_t bytes)
-{
-  if (g_ctx.staging_cap >= bytes) return QGB_OK;
-  if (g_ctx.staging) cudaFree(g_ctx.staging);
-  g_ctx.staging = nullptr;
-  g_ctx.staging_cap = 0;
-  QGB_TRY_CUDA(cudaMalloc(&g_ctx.staging, bytes));
-  g_ctx.staging_cap = bytes;
-  return QGB_OK;
-}
-
-// Reusable device buffers of a given size; `tag` distinguishes simultaneous uses.
-int get_scratch(size_t bytes, int tag, void** out)
-{
-  auto& v = g_ctx.scratch[std::make_pair(bytes, tag)];
-  if (v.empty()) {
-    void* p = nullptr;
-    QGB_TRY_CUDA(cudaMalloc(&p, bytes));
-    v.push_back(p);
-    // zero once: scratch buffers can become a field's storage (flow_step swaps
-    // them), and the padding sites of every field stay zero
-    QGB_TRY_CUDA(cudaMemsetAsync(p, 0, bytes, g_ctx.stream));
-  }
-  *out = v[0];
-  return QGB_OK;
-}
-
 // The flow adjoint's fields: the states at the checkpoints, the links before each
 // step of a segment, and the stage fields of those steps (5 j + k: the links
 // after stages 1 and 2 and the three stages' Z).
 enum AdjField { ADJ_CHECKPOINT, ADJ_LINKS, ADJ_STAGE };
-
-int adj_field(size_t bytes, AdjField what, int index, void** out)
-{
-  void*& p = g_ctx.adjoint[std::make_tuple(bytes, (int)what, index)];
-  if (!p) {
-    const cudaError_t e = cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) p = nullptr;
-    QGB_TRY_CUDA(e);
-    QGB_TRY_CUDA(cudaMemsetAsync(p, 0, bytes, g_ctx.stream));  // the padding sites stay zero, as in get_scratch
-  }
-  *out = p;
-  return QGB_OK;
-}
 
 // Frees the adjoint's fields but the first n[what] of each kind with `bytes` bytes (no recorded graph uses them).
 void release_adjoint_fields(int64_t* released, size_t bytes = 0, const int* n = nullptr)
@@ -317,6 +267,79 @@ void release_field_pool()
     for (void* p : kv.second) cudaFree(p);
   g_ctx.field_pool.clear();
   g_ctx.field_pool_bytes = 0;
+}
+
+// Gives back the memory that nothing uses: destroyed fields' storage, the adjoint's fields between its calls and the
+// work pool's.  Adds the bytes to *released.
+void release_idle_memory(int64_t* released)
+{
+  if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
+  if (released) *released += (int64_t)g_ctx.field_pool_bytes;
+  release_field_pool();
+  if (!g_ctx.adjoint_busy) release_adjoint_fields(released);
+  qgb::trim_work_pool(released);
+}
+
+// cudaMalloc, tried again without the library's idle memory when the device has run out.
+cudaError_t device_alloc(void** p, size_t bytes)
+{
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    release_idle_memory(nullptr);
+    e = cudaMalloc(p, bytes);
+  }
+  if (e != cudaSuccess) *p = nullptr;
+  return e;
+}
+
+int ensure_partials(size_t n)
+{
+  if (g_ctx.partials_cap >= n) return QGB_OK;
+  if (g_ctx.partials) cudaFree(g_ctx.partials);
+  g_ctx.partials = nullptr;
+  g_ctx.partials_cap = 0;
+  QGB_TRY_CUDA(device_alloc((void**)&g_ctx.partials, n * sizeof(double)));
+  g_ctx.partials_cap = n;
+  return QGB_OK;
+}
+
+int ensure_staging(size_t bytes)
+{
+  if (g_ctx.staging_cap >= bytes) return QGB_OK;
+  if (g_ctx.staging) cudaFree(g_ctx.staging);
+  g_ctx.staging = nullptr;
+  g_ctx.staging_cap = 0;
+  QGB_TRY_CUDA(device_alloc((void**)&g_ctx.staging, bytes));
+  g_ctx.staging_cap = bytes;
+  return QGB_OK;
+}
+
+// Reusable device buffers of a given size; `tag` distinguishes simultaneous uses.
+int get_scratch(size_t bytes, int tag, void** out)
+{
+  auto& v = g_ctx.scratch[std::make_pair(bytes, tag)];
+  if (v.empty()) {
+    void* p = nullptr;
+    QGB_TRY_CUDA(device_alloc(&p, bytes));
+    v.push_back(p);
+    // zero once: scratch buffers can become a field's storage (flow_step swaps
+    // them), and the padding sites of every field stay zero
+    QGB_TRY_CUDA(cudaMemsetAsync(p, 0, bytes, g_ctx.stream));
+  }
+  *out = v[0];
+  return QGB_OK;
+}
+
+int adj_field(size_t bytes, AdjField what, int index, void** out)
+{
+  void*& p = g_ctx.adjoint[std::make_tuple(bytes, (int)what, index)];
+  if (!p) {
+    QGB_TRY_CUDA(device_alloc(&p, bytes));
+    QGB_TRY_CUDA(cudaMemsetAsync(p, 0, bytes, g_ctx.stream));  // the padding sites stay zero, as in get_scratch
+  }
+  *out = p;
+  return QGB_OK;
 }
 
 int read_results(int slot, int n, double* out)
@@ -929,6 +952,7 @@ struct AdjPlan {
   int every = 0;         // steps of a segment
   std::vector<void*> cps, links, stages;  // checkpoints (none with `all`), a segment's links and stage fields
   void* w[10];                            // work fields
+  ~AdjPlan() { g_ctx.adjoint_busy = false; }
 };
 
 static bool adj_fits(size_t bytes, int steps, size_t bound) { return (size_t)steps <= bound / (6 * bytes); }
@@ -965,18 +989,20 @@ static int adj_fields(size_t bytes, AdjField what, int n, std::vector<void*>* ou
 }
 
 // The buffers for a flow of `steps` steps with a checkpoint every `every` of them (not used where the whole flow is
-// kept).  What does not fit the bounds or the device is recomputed, which changes at most rounding.
+// kept).  What does not fit the bounds or the device is recomputed, which changes at most rounding.  The adjoint's
+// fields are the call's until *p goes.
 static int adj_plan(size_t bytes, int steps, int every, AdjPlan* p)
 {
   for (int i = 0; i < 10; ++i) QGB_RC(get_scratch(bytes, 41 + i, &p->w[i]));
   if (adj_fits(bytes, steps, g_adj_flow_bytes)) {
     const int n[3] = {0, steps, 5 * steps};
     if (adj_room(bytes, n)) {
+      g_ctx.adjoint_busy = true;
       p->every = steps;
       p->all = p->segment = adj_fields(bytes, ADJ_LINKS, steps, &p->links) == QGB_OK &&
                             adj_fields(bytes, ADJ_STAGE, 5 * steps, &p->stages) == QGB_OK;
       if (p->all) return QGB_OK;
-      (void)cudaGetLastError();
+      g_ctx.adjoint_busy = false;
       release_adjoint_fields(nullptr);
     }
   }
@@ -984,12 +1010,12 @@ static int adj_plan(size_t bytes, int steps, int every, AdjPlan* p)
     void* t = nullptr;
     QGB_RC(get_scratch(bytes, 21 + i, &t));
   }
+  g_ctx.adjoint_busy = true;
   int n[3] = {(steps - 1) / every + 1, every, 0};
   p->every = every;
   if (adj_fits(bytes, every, g_adj_segment_bytes)) {
     n[ADJ_STAGE] = 5 * every;
     p->segment = adj_room(bytes, n) && adj_fields(bytes, ADJ_STAGE, 5 * every, &p->stages) == QGB_OK;
-    (void)cudaGetLastError();
   }
   if (!p->segment) {
     n[ADJ_STAGE] = 0;
@@ -1135,16 +1161,19 @@ int force_on(const Geo& g, const void* U, void* out, double beta, double c1)
   QGB_CTX();
   return force<double>(g, FORCE_SET, fargs(U, out, beta, c1, 0.0));
 }
-cudaError_t work_pool(cudaMemPool_t* out)
+// The device's pool for work buffers.  It keeps at most 1 GiB from call to call; beyond that the memory goes back to
+// the device when a stream is next synchronised.
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pools[64] = {};
+
+static cudaError_t work_pool(cudaMemPool_t* out)
 {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (dev >= 64) return cudaErrorInvalidDevice;
-  std::lock_guard<std::mutex> lock(mu);
-  if (!pools[dev]) {
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  if (!g_pools[dev]) {
     cudaMemPoolProps props;
     memset(&props, 0, sizeof(props));
     props.allocType = cudaMemAllocationTypePinned;
@@ -1156,10 +1185,48 @@ cudaError_t work_pool(cudaMemPool_t* out)
     uint64_t keep = (uint64_t)1 << 30;
     e = cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
     if (e != cudaSuccess) return e;
-    pools[dev] = p;
+    g_pools[dev] = p;
   }
-  *out = pools[dev];
+  *out = g_pools[dev];
   return cudaSuccess;
+}
+
+void trim_work_pool(int64_t* released)
+{
+  std::lock_guard<std::mutex> lock(g_pool_mu);
+  for (cudaMemPool_t p : g_pools) {
+    if (!p) continue;
+    uint64_t before = 0, after = 0;
+    cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &before);
+    cudaMemPoolTrimTo(p, 0);
+    cudaMemPoolGetAttribute(p, cudaMemPoolAttrReservedMemCurrent, &after);
+    if (released) *released += (int64_t)(before - after);
+  }
+}
+
+cudaError_t work_alloc(void** p, size_t bytes, cudaStream_t st)
+{
+  cudaMemPool_t pool = nullptr;
+  cudaError_t e = work_pool(&pool);
+  if (e == cudaSuccess) e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, st);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    std::lock_guard<std::recursive_mutex> lock(g_mu);
+    release_idle_memory(nullptr);
+    e = cudaMallocFromPoolAsync(p, bytes > 0 ? bytes : 1, pool, st);
+  }
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
+
+// cudaMalloc for the other units, with device_alloc's second try.
+cudaError_t alloc_or_release(void** p, size_t bytes)
+{
+  std::lock_guard<std::recursive_mutex> lock(g_mu);
+  return device_alloc(p, bytes);
 }
 // Lets the allocation-free entry point (noalloc.cu) report through qgb_last_error.
 void set_last_error(const std::string& msg) { g_err = msg; }
@@ -1276,14 +1343,7 @@ int qgb_field_create(qgb_field** out, const int32_t total_site[4], int32_t multi
     pooled->second.pop_back();
     g_ctx.field_pool_bytes -= f->bytes;
   } else {
-    e = cudaMalloc(&f->d, f->bytes);
-    if (e == cudaErrorMemoryAllocation) {
-      cudaGetLastError();
-      cudaStreamSynchronize(g_ctx.stream);
-      release_field_pool();
-      release_adjoint_fields(nullptr);
-      e = cudaMalloc(&f->d, f->bytes);
-    }
+    e = device_alloc((void**)&f->d, f->bytes);
   }
   if (e != cudaSuccess) {
     delete f;
@@ -1319,10 +1379,8 @@ int qgb_field_destroy(qgb_field* f)
 int qgb_field_pool_release(int64_t* released)
 {
   std::lock_guard<std::recursive_mutex> lock(g_mu);
-  if (released) *released = (int64_t)g_ctx.field_pool_bytes;
-  if (g_ctx.ready) cudaStreamSynchronize(g_ctx.stream);
-  release_field_pool();
-  release_adjoint_fields(released);
+  if (released) *released = 0;
+  release_idle_memory(released);
   return QGB_OK;
 }
 
@@ -1399,7 +1457,7 @@ static int up_start(int i, const double* host, size_t bytes)
     if (g_ctx.up_buf[i]) QGB_TRY_CUDA(cudaFree(g_ctx.up_buf[i]));
     g_ctx.up_buf[i] = nullptr;
     g_ctx.up_cap[i] = 0;
-    QGB_TRY_CUDA(cudaMalloc(&g_ctx.up_buf[i], bytes));
+    QGB_TRY_CUDA(device_alloc(&g_ctx.up_buf[i], bytes));
     g_ctx.up_cap[i] = bytes;
   }
   QGB_TRY_CUDA(cudaEventRecord(g_ctx.up_order[i], g_ctx.stream));
@@ -1467,7 +1525,7 @@ int qgb_field_download_async(const qgb_field* f, double* host)
     if (g_ctx.dn_buf[i]) QGB_TRY_CUDA(cudaFree(g_ctx.dn_buf[i]));
     g_ctx.dn_buf[i] = nullptr;
     g_ctx.dn_cap[i] = 0;
-    QGB_TRY_CUDA(cudaMalloc(&g_ctx.dn_buf[i], bytes));
+    QGB_TRY_CUDA(device_alloc(&g_ctx.dn_buf[i], bytes));
     g_ctx.dn_cap[i] = bytes;
   }
   QGB_RC(download_to_device_aos(f, (double*)g_ctx.dn_buf[i]));

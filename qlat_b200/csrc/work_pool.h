@@ -6,10 +6,13 @@
 namespace qgb
 {
 
-// The device's pool for work buffers (capi.cu).  It keeps at most 1 GiB from
-// call to call; beyond that the memory goes back to the device when a stream
-// is next synchronised.
-cudaError_t work_pool(cudaMemPool_t* out);
+// A work buffer of the device's pool (capi.cu); when the device has run out, tried again without the library's idle
+// memory.
+cudaError_t work_alloc(void** p, size_t bytes, cudaStream_t st);
+// Returns the pool's unused memory to the device; adds the bytes to *released.
+void trim_work_pool(int64_t* released);
+// cudaMalloc with that second try.
+cudaError_t alloc_or_release(void** p, size_t bytes);
 
 // A buffer of the work pool, freed in stream order when it goes out of scope.
 // Each call owns its buffers, so calls of several threads share none.
@@ -25,12 +28,8 @@ struct WorkBuf {
   }
   cudaError_t alloc(size_t bytes, cudaStream_t stream)
   {
-    cudaMemPool_t pool = nullptr;
-    cudaError_t e = work_pool(&pool);
     st = stream;
-    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&p, bytes > 0 ? bytes : 1, pool, stream);
-    if (e != cudaSuccess) p = nullptr;
-    return e;
+    return work_alloc(&p, bytes, stream);
   }
 };
 

@@ -61,3 +61,32 @@ def test_transfer_without_room_leaves_the_next_ones_usable(q):
         b.from_numpy(big)
         assert np.array_equal(b.to_numpy(), big) and np.array_equal(a.to_numpy(), small)
     ''')
+
+
+@pytest.mark.gpu
+def test_idle_memory_is_given_up_for_every_kind_of_buffer(q):
+    """The flow adjoint holds 9 GB for its next call and the device has 64 MB left: staging, work fields of a trajectory,
+    the work pool, fields, and batches find room all the same, each with the buffers held anew."""
+    run(q, '''
+        g, big = links((16, 16, 16, 16)), links((16, 16, 16, 32))
+        gm, F = q.GaugeMomentum(big.geo), q.GaugeMomentum(big.geo)
+        gm.set_rand(q.RngState("memory"), 1.0)
+        ga, fi = q.GaugeAction(5.5, 0.0), q.FlowInfo([q.FlowStepInfo(1, 0, 0.1, 1)])
+        want = q.gf_flow_action_grad(g, 0.01, 40, 5.5)
+        made = []
+        for use in (lambda: q.run_hmc_evolve_pure_gauge(gm, big, ga, None, 1, 0.1, integrator="leapfrog"),
+                    lambda: q.set_gm_force_flowed(F, big, ga, fi),
+                    lambda: made.append(q.ChainBatch([(8, 8, 8, 8)] * 64, [5.5] * 64)),
+                    lambda: made.append(big.copy()),
+                    lambda: big.to_numpy()):
+            q.gf_flow_action_grad(g, 0.01, 40, 5.5)
+            with Filled(64 << 20):
+                use()
+                assert torch.cuda.mem_get_info()[0] > 7 << 30  # what the adjoint held and the call did not take
+        # a short device cannot take the fields of a running gradient from it
+        with Filled(3 << 30):
+            loss, grad = q.gf_flow_action_grad(g, 0.01, 40, 5.5)
+        assert loss == want[0] and np.array_equal(np.asarray(grad), np.asarray(want[1]))
+        # and the work pool is given back too
+        assert q.release_field_pool() > 0 and q.release_field_pool() == 0
+    ''')
