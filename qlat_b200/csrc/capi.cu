@@ -431,8 +431,11 @@ int topology_5li_slot(const qgb_field* gf, qgb_field* terms, qgb_field* total, i
   const int nb = qgb::clover_blocks(g);
   QGB_RC(ensure_partials((size_t)nb * 5));
   qgb::WorkBuf lines;
-  QGB_TRY_CUDA(lines.alloc(qgb::lines_bytes(g, gf->prec == QGB_F64 ? 8 : 4), g_ctx.stream));
-  Prof p("topology_5li", 3);
+  // the lines of two and three links, twice the gauge field; without room for them the kernel forms them where it
+  // reads them
+  const cudaError_t e = lines.alloc(qgb::lines_bytes(g, gf->prec == QGB_F64 ? 8 : 4), g_ctx.stream);
+  if (e != cudaErrorMemoryAllocation) QGB_TRY_CUDA(e);
+  Prof p("topology_5li", lines.p ? 3 : 2);
   if (gf->prec == QGB_F64)
     QGB_TRY_CUDA(qgb::launch_topology_5li<double>(g, gf->d, lines.p, terms ? terms->d : nullptr, total ? total->d : nullptr,
                                                   g_ctx.partials, g_ctx.stream));

@@ -100,9 +100,9 @@ __device__ __forceinline__ M3<R> sub_adj_mul(const M3<R>& s, const M3<R>& a, con
 }
 
 // acc += G at site s; m and n links: am, bn (and amm, bnn) lead m links along a (n along b) forward (backward).
-template <typename R, typename I>
-__device__ __forceinline__ void add_leaves(M3<R>& acc, const CompLd<R, I>& A, const CompLd<R, I>& B, I s, I am, I amm, I bn,
-                                           I bnn)
+// A, B: CompLd, or LineWalk.
+template <typename R, typename I, typename Line>
+__device__ __forceinline__ void add_leaves(M3<R>& acc, const Line& A, const Line& B, I s, I am, I amm, I bn, I bnn)
 {
 #pragma unroll 1
   for (int h = 0; h < 2; ++h) {
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3) k_clover(Geo g, co
       const int xa = sel4(x.c, a), xb = sel4(x.c, b), La = sel4(g.d, a), Lb = sel4(g.d, b);
       const I sa = site_stride<I>(g, a), sb = site_stride<I>(g, b);
       M3<R> G = m3_zero<R>();
-      add_leaves<R, I>(G, CompLd<R, I>{Up + a * comp}, CompLd<R, I>{Up + b * comp}, s, nb_offset<I>(xa, 1, La, sa),
+      add_leaves(G, CompLd<R, I>{Up + a * comp}, CompLd<R, I>{Up + b * comp}, s, nb_offset<I>(xa, 1, La, sa),
                        nb_offset<I>(xa, -1, La, sa), nb_offset<I>(xb, 1, Lb, sb), nb_offset<I>(xb, -1, Lb, sb));
       const AntiH<R> f = antiherm(R(0.125), G);
       e += (double)energy_of(f);
@@ -233,12 +233,31 @@ __global__ void __launch_bounds__(128) k_lines(Geo g, const Cx<R>* Up, Cx<R>* li
   L.st(s, 4 + a, mul(d, U((I)s + nb_offset<I>(xa, 2, La, sa))));
 }
 
+// The line of m links along a direction of extent L from site y, formed from its links as k_lines does: what
+// k_topology_5li reads where the device has no room for the lines (1.2 KB a site in FP64).  1092 links a site from L2
+// instead of 588 lines, and the products of each line again: 16^3 x 32 2.22 ms in FP64 against 0.64, 24^3 x 48 23.2
+// against 3.24.
+template <typename R, typename I>
+struct LineWalk {
+  CompLd<R, I> U;
+  int m, L;
+  I stride;
+  __device__ __forceinline__ M3<R> operator()(I y) const
+  {
+    const int x = (int)((y / stride) % L);
+    M3<R> r = U(y);
+#pragma unroll 1
+    for (int i = 1; i < m; ++i) r = mul(r, U(y + nb_offset<I>(x, i, L, stride)));
+    return r;
+  }
+};
+
 // The five terms c_k / (m n)^2 q_{m x n} of the improved charge, (m, n) = (1,1), (2,2), (1,2), (1,3), (3,3), the
 // unequal ones averaged with their transposes (qcd.cpp:536-568): terms (multiplicity 5) and total (multiplicity
 // 1) fields, each optional, and the block sums of the terms.
 // 420 products per site and the 8 of k_lines, where walking every loop link by link took 1080; 16^3 x 32,
 // FP64: 2.71 -> 0.60 ms, and 0.04 ms for the lines.
-template <typename R, typename I>
+template <typename R, typename I, bool LINES>
 __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
     k_topology_5li(Geo g, const Cx<R>* Up, const Cx<R>* lines, R* terms, R* total, double* partials)
 {
@@ -251,7 +270,10 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
   {
     const Coord x = coord_of(g, site);
     const I comp = (I)site_blocks(g.V) * 288, s = (I)site;
-    auto line = [&](int a, int m) { return CompLd<R, I>{(m == 1 ? Up : lines + (m == 3 ? 4 * comp : (I)0)) + a * comp}; };
+    auto line = [&](int a, int m) {
+      if constexpr (LINES) return CompLd<R, I>{(m == 1 ? Up : lines + (m == 3 ? 4 * comp : (I)0)) + a * comp};
+      else return LineWalk<R, I>{CompLd<R, I>{Up + a * comp}, m, sel4(g.d, a), site_stride<I>(g, a)};
+    };
 #pragma unroll 1
     for (int k = 0; k < 5; ++k) {
       const int m0 = k == 1 ? 2 : (k == 4 ? 3 : 1), n0 = k == 0 ? 1 : (k == 1 || k == 2 ? 2 : 3);
@@ -266,7 +288,7 @@ __global__ void __launch_bounds__(BS, sizeof(R) == 8 ? 2 : 3)
 #pragma unroll 1
         for (int h = 0; h <= (m0 != n0); ++h) {
           const int m = h == 0 ? m0 : n0, n = h == 0 ? n0 : m0;
-          add_leaves<R, I>(G, line(a, m), line(b, n), s, nb_offset<I>(xa, m, La, sa), nb_offset<I>(xa, -m, La, sa),
+          add_leaves(G, line(a, m), line(b, n), s, nb_offset<I>(xa, m, La, sa), nb_offset<I>(xa, -m, La, sa),
                            nb_offset<I>(xb, n, Lb, sb), nb_offset<I>(xb, -n, Lb, sb));
         }
         const AntiH<R> f = antiherm(m0 == n0 ? R(0.125) : R(0.0625), G);
@@ -325,14 +347,21 @@ cudaError_t launch_topology_5li(const Geo& g, const void* U, void* lines, void* 
                                 cudaStream_t st)
 {
   const dim3 grid((unsigned)((g.V + 127) / 128), 4);
-  if (small_offsets(g, 8)) {
-    k_lines<R, int><<<grid, 128, 0, st>>>(g, (const Cx<R>*)U, (Cx<R>*)lines);
-    k_topology_5li<R, int><<<clover_blocks(g), BS, 0, st>>>(g, (const Cx<R>*)U, (const Cx<R>*)lines, (R*)terms,
-                                                            (R*)total, partials);
+  const Cx<R>* u = (const Cx<R>*)U;
+  Cx<R>* l = (Cx<R>*)lines;
+  auto sums = [&](auto kernel) {
+    kernel<<<clover_blocks(g), BS, 0, st>>>(g, u, (const Cx<R>*)l, (R*)terms, (R*)total, partials);
+  };
+  if (lines == nullptr && small_offsets(g, 4)) {
+    sums(k_topology_5li<R, int, false>);
+  } else if (lines == nullptr) {
+    sums(k_topology_5li<R, long, false>);
+  } else if (small_offsets(g, 8)) {
+    k_lines<R, int><<<grid, 128, 0, st>>>(g, u, l);
+    sums(k_topology_5li<R, int, true>);
   } else {
-    k_lines<R, long><<<grid, 128, 0, st>>>(g, (const Cx<R>*)U, (Cx<R>*)lines);
-    k_topology_5li<R, long><<<clover_blocks(g), BS, 0, st>>>(g, (const Cx<R>*)U, (const Cx<R>*)lines, (R*)terms,
-                                                             (R*)total, partials);
+    k_lines<R, long><<<grid, 128, 0, st>>>(g, u, l);
+    sums(k_topology_5li<R, long, true>);
   }
   return cudaGetLastError();
 }

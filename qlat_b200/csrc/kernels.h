@@ -199,7 +199,7 @@ cudaError_t launch_clover(const Geo& g, const void* U, void* e_field, void* q_fi
                           cudaStream_t st);
 // values 0..4: the five terms of the 5-loop improved charge (qcd.cpp:425-489);
 // optional fields: terms (real, multiplicity 5) and their per-site sum (multiplicity 1);
-// lines: work buffer of lines_bytes(g, sizeof(R)) bytes
+// lines: work buffer of lines_bytes(g, sizeof(R)) bytes, or null: the same sums without it, slower
 size_t lines_bytes(const Geo& g, size_t real);
 template <typename R>
 cudaError_t launch_topology_5li(const Geo& g, const void* U, void* lines, void* terms, void* total, double* partials,

@@ -90,3 +90,30 @@ def test_idle_memory_is_given_up_for_every_kind_of_buffer(q):
         # and the work pool is given back too
         assert q.release_field_pool() > 0 and q.release_field_pool() == 0
     ''')
+
+
+@pytest.mark.gpu
+def test_improved_charge_needs_no_room(q):
+    """The five loops' terms with and without room for the field of lines (1.2 KB a site in FP64): the same products
+    in the same order.  Extents of 1 to 3 (lines that wrap around) and partly filled blocks of 64 sites."""
+    run(q, '''
+        from qlat_b200._lib import call
+        for ts in ((16, 16, 16, 32), (1, 2, 3, 20000), (17, 15, 19, 20)):
+            for precision in (q.F64, q.F32):
+                gf = links(ts).copy(precision=precision)
+                topf = q.FieldRealD(gf.geo, 5, precision=precision)
+                out = []
+                for spare in (None, 24 << 20):  # (the lines are 55 to 151 MB)
+                    q.release_field_pool()
+                    n0 = q.launch_count()
+                    if spare is None:
+                        out.append(q.gf_topology_terms(gf))
+                    else:
+                        with Filled(spare):
+                            out.append(q.gf_topology_terms(gf))
+                            call("qgb_clf_topology_field_5_terms", topf.handle, gf.handle)
+                    out.append(q.launch_count() - n0)
+                assert out[1] == 3 and out[3] == 4, "three kernels with the lines, two without"
+                assert np.array_equal(out[0], out[2]), (ts, precision, out)
+                assert np.array_equal(np.asarray(topf), np.asarray(q.gf_topology_terms_field(gf)))
+    ''')
