@@ -82,10 +82,11 @@ int qgb_field_create(qgb_field** out, const int32_t total_site[4], int32_t multi
  * run_hmc_pure_gauge, hmc.pyx:190-216, builds a link copy and a momentum field
  * every trajectory). */
 int qgb_field_destroy(qgb_field* f);
-/* Frees the pooled storage of destroyed fields and the checkpoints and stage
- * fields that the flow adjoint keeps for its next call (qgb_field_create also
- * does this by itself when cudaMalloc runs out of memory); writes the bytes
- * freed when released is not NULL. */
+/* Frees what the library holds for later calls: the storage of destroyed
+ * fields, the fields that the flow adjoint keeps, the work buffers' pool (at
+ * most 1 GiB) and the packed fields of FP32 rectangle forces (with the recorded
+ * trajectories).  Writes the bytes freed when released is not NULL.  An
+ * allocation that fails frees all but the last by itself and tries again. */
 int qgb_field_pool_release(int64_t* released);
 /* Bounds on the fields that the flow adjoint keeps, six per step, and holds for
  * its next call: of a whole flow, also over all lattices together (10 GiB; 0:

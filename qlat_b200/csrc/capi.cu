@@ -524,7 +524,10 @@ struct PairFields {
   void *u = nullptr, *t = nullptr, *p = nullptr;  // links, a second link buffer, momenta (or Z)
 };
 
+const int PAIR_TAG = 71;  // of get_scratch: u, t, p
 const long MIN_PAIRS = 16384;  // below, half as many threads leave the GPU idle: 8^4, 0.61 ms in pairs against 0.52
+
+void drop_traj_graphs();
 
 // The packed fields of lattice g; false when it cannot be packed, is too small, or the device has no room for
 // them (the scalar form then runs as it did without).
@@ -533,11 +536,11 @@ bool pair_fields(const Geo& g, PairFields* f)
   if (!qgb::pair_geo(g, &f->pg) || f->pg.pairs < MIN_PAIRS) return false;
   void** slots[3] = {&f->u, &f->t, &f->p};
   for (int i = 0; i < 3; ++i)
-    if (get_scratch(f->pg.bytes, 71 + i, slots[i]) != QGB_OK) {
+    if (get_scratch(f->pg.bytes, PAIR_TAG + i, slots[i]) != QGB_OK) {
       (void)cudaGetLastError();
       for (int j = 0; j < i; ++j) {  // no recorded graph can hold a part of the set
         cudaFree(*slots[j]);
-        g_ctx.scratch.erase(std::make_pair(f->pg.bytes, 71 + j));
+        g_ctx.scratch.erase(std::make_pair(f->pg.bytes, PAIR_TAG + j));
       }
       return false;
     }
@@ -584,6 +587,25 @@ bool use_pairs(const Geo& g, double c1, int forces, int passes, PairFields* f)
 
 // force launches of md_trajectory
 int md_forces(int integrator, int n_step) { return integrator == QGB_INTEGRATOR_FORCE_GRADIENT ? 4 * n_step : n_step; }
+
+// Frees the packed fields of all lattices and the recorded trajectories, which may hold them (between calls only).
+void release_pair_fields(int64_t* released)
+{
+  bool any = false;
+  for (auto it = g_ctx.scratch.begin(); it != g_ctx.scratch.end();) {
+    if (it->first.second < PAIR_TAG || it->first.second > PAIR_TAG + 2) {
+      ++it;
+      continue;
+    }
+    for (void* p : it->second) {
+      cudaFree(p);
+      *released += (int64_t)it->first.first;
+      any = true;
+    }
+    it = g_ctx.scratch.erase(it);
+  }
+  if (any) drop_traj_graphs();
+}
 
 int pair_pack(const Geo& g, const PairFields& f, const void* natural, void* packed)
 {
@@ -1382,8 +1404,10 @@ int qgb_field_destroy(qgb_field* f)
 int qgb_field_pool_release(int64_t* released)
 {
   std::lock_guard<std::recursive_mutex> lock(g_mu);
-  if (released) *released = 0;
-  release_idle_memory(released);
+  int64_t n = 0;
+  release_idle_memory(&n);
+  release_pair_fields(&n);
+  if (released) *released = n;
   return QGB_OK;
 }
 

@@ -132,3 +132,24 @@ def test_autotuner_times_the_paired_shape(q):
     assert n == 2  # its links and momenta, packed for the timing
     assert 0 <= best[0] < len(q.force_variants()) and ms[0] > 0
     q.force_set_variant(q.F32, True, old)
+
+
+@pytest.mark.gpu
+def test_packed_fields_are_given_back(q):
+    ts = (16, 16, 16, 16)
+    gf, gm = start(q, ts)
+    ga = q.GaugeAction(2.13, -0.331)
+    keep = []
+
+    def traj():
+        u, p = gf.copy(), gm.copy()
+        keep.extend((u, p))  # (so that they do not go to the field pool)
+        dh = q.run_hmc_evolve_pure_gauge(p, u, ga, None, 8, precision="mixed")
+        return np.asarray(u), np.asarray(p), dh
+
+    q.release_field_pool()
+    want = [traj() for _ in range(3)][-1]
+    # links, links, momenta: t of 8 + 4 pairs instead of 16 sites, two sites each
+    assert q.release_field_pool() >= 3 * 4 * 16 ** 3 * 12 * 2 * 72
+    for got in [traj() for _ in range(3)]:
+        assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1]) and got[2] == want[2]
