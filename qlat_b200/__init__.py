@@ -163,9 +163,10 @@ def download_join():
 
 
 def release_field_pool() -> int:
-    """Free the device storage the library keeps from destroyed fields for
-    reuse (torch.cuda.empty_cache for this library's fields); returns the
-    bytes freed."""
+    """Free the device memory the library holds for later calls: destroyed
+    fields' storage, the flow adjoint's kept fields, the work pool and the packed
+    fields of FP32 rectangle forces (torch.cuda.empty_cache for this library);
+    returns the bytes freed."""
     import ctypes
     from ._lib import call
     n = ctypes.c_int64()

@@ -153,8 +153,8 @@ struct SmemAcc {
 // links give
 //   +nu: dV = Y_H V + H (Y_M W - W Y_K)
 //   -nu: dV = H^+ ((Y_M - Y_H) W + M (Y_K K))
-// 6 products per direction, 3 of them with an anti-Hermitian factor, where dual matrices
-// (k_force_vjp_rect) take 9 full ones: the kernel is bound by the FP64 pipe, 3900 multiply-adds per link
+// 6 products per direction, 3 of them with an anti-Hermitian factor along +nu and 2 along -nu, where dual
+// matrices (k_force_vjp_rect) take 9 full ones: the kernel is bound by the FP64 pipe, 3900 multiply-adds per link
 // instead of 6600.  S and dS accumulate in shared memory, which leaves the registers to the products
 // (3 blocks of 128 threads per SM).  The four directions of a site block run back to back and meet in L2.
 // 16^4 FP64: 0.188 -> 0.112 ms a launch.

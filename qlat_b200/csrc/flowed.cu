@@ -285,7 +285,7 @@ __device__ __forceinline__ double gauss8(double (&m)[8], double (&inv)[8], int b
 // both the reference's order-20 polynomials, cut once the omitted terms are below 2^-58 of the sum.
 // One thread per link held all of it in local memory and differentiated J eight times over: 2.57 ms
 // a step on 8^3 x 16 (with the staple's own launch, 2.58), against 35 us (size 1) and 27 us (size 2) here.
-// At 4096 links it is bound by the latency of its chains (4 warps' worth of links per SM), not by FP64 rate.
+// At 4096 links (1024 warps: 8 on each of 128 SMs) it is bound by the latency of its chains, not by FP64 rate.
 template <int SZ, int MODE>
 __global__ void __launch_bounds__(FLOW_BS) k_flow_step(FlowArgs a)
 {

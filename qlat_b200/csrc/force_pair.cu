@@ -12,11 +12,13 @@
 //
 // At 255 registers a thread carries the staple's matrices of both sites
 // without spills, 8 warps per SM.  Iwasaki force + momentum + link update at
-// 24^3 x 64: 1.17 ms in the scalar two-row form (435 M warp instructions at
-// half this size, 0.8 no_instruction stalls per issue) against 0.99 ms (222 M,
-// 0.06), and 8 force-gradient steps 38.9 against 35.0 ms.  Three or four blocks
-// per SM spill or take shared memory from L1: 1.19 to 2.0 ms a launch.  The
-// plaquette force gains 4% and stays scalar.
+// 24^3 x 48: 675 M warp instructions and 1.2 no_instruction stalls per issue in
+// the scalar two-row form, 345 M and 0.06 here; at 24^3 x 64 a force launch of
+// a trajectory takes 1.16 against 1.03 ms (both kinds of launch of the
+// force-gradient step averaged), and 8 such steps 38.9 against 35.0 ms.  Three
+// or four blocks per SM spill or take shared memory from L1: 1.19 to 2.0 ms a
+// launch.  The plaquette force gains 4% and stays scalar.  capi.cu:pairs_pay
+// says which runs go in pairs.
 #include "force_impl.cuh"
 #include "pair.cuh"
 

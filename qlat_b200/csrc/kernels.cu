@@ -675,8 +675,8 @@ __global__ void __launch_bounds__(128) k_hot_start_batch(long Vtot, int nchain, 
 // Site values for the per-chain Hamiltonians.
 
 // vals[sg] = sum_mu -tr(P^2)/2, and with COPY the momenta converted to RO into Q in the same pass (padded sites
-// included, with the zeros of P's).  Memory-bound: 1.69 M sites (256 chains of 4^4 to 12^4), 0.21 ms with the copy and
-// 0.05 ms from FP32.
+// included, with the zeros of P's).  Memory-bound: 1.69 M sites (256 chains of 4^4 to 12^4) in a trajectory, 0.220 ms
+// with the copy (1.47 GB) and 0.062 ms from FP32 (0.50 GB, of which the L2 still holds what the last force wrote).
 template <typename RI, typename RO, bool COPY>
 __global__ void __launch_bounds__(256) k_batch_kinetic(long Vtot, const Cx<RI>* P, Cx<RO>* Q, double* vals)
 {
