@@ -703,13 +703,16 @@ __global__ void __launch_bounds__(256) k_batch_kinetic(long Vtot, const Cx<RI>* 
 
 // Plaquette sums into vals[sg] and, with RECT, rectangle sums into vals[Vtot + sg], as k_action_corners within
 // each site's chain (8 products per plane instead of 10 from 64-bit index walks); with copy != nullptr also the
-// links in FP32 (padded sites included).
+// links in FP32 (padded sites included).  Blocks of 64 sites, so that a small batch spreads over the SMs: one chain of
+// 4^4 8.9 -> 7.8 us, three of 4^4 to 8^4 with rectangles 23.7 -> 17.7 (blocks of 256 before), 256 chains as before.
+constexpr int ACT_BS = 64;
+
 template <bool RECT>
-__global__ void __launch_bounds__(256, RECT ? 1 : 2)
+__global__ void __launch_bounds__(ACT_BS, RECT ? 4 : 8)
     k_batch_action(long Vtot, int nchain, const long* __restrict__ offs, const ChainInfo* __restrict__ chains,
                    const Cx<double>* U, Cx<float>* copy, double* vals)
 {
-  const long sg = (long)blockIdx.x * 256 + threadIdx.x;
+  const long sg = (long)blockIdx.x * ACT_BS + threadIdx.x;
   if (copy != nullptr && sg < padded_sites(Vtot)) {
     const CField<double> Uf{U, Vtot};
 #pragma unroll 1
@@ -861,9 +864,9 @@ cudaError_t launch_batch_action(long Vtot, int nchain, const long* offs, const C
   const Cx<double>* u = (const Cx<double>*)U;
   Cx<float>* c = (Cx<float>*)copy_f32;
   if (padded_sites(Vtot) * 36 < 2147483647L) {
-    const unsigned grid = (unsigned)((padded_sites(Vtot) + 255) / 256);
-    if (rect) k_batch_action<true><<<grid, 256, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
-    else k_batch_action<false><<<grid, 256, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
+    const unsigned grid = (unsigned)((padded_sites(Vtot) + ACT_BS - 1) / ACT_BS);
+    if (rect) k_batch_action<true><<<grid, ACT_BS, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
+    else k_batch_action<false><<<grid, ACT_BS, 0, st>>>(Vtot, nchain, offs, chains, u, c, vals);
     return cudaGetLastError();
   }
   k_batch_action_large<double><<<(unsigned)((Vtot + 127) / 128), 128, 0, st>>>(Vtot, nchain, offs, chains, rect, u, vals);
