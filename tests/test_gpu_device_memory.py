@@ -117,3 +117,51 @@ def test_improved_charge_needs_no_room(q):
                 assert np.array_equal(out[0], out[2]), (ts, precision, out)
                 assert np.array_equal(np.asarray(topf), np.asarray(q.gf_topology_terms_field(gf)))
     ''')
+
+
+@pytest.mark.gpu
+def test_pairs_of_sites_without_room_run_in_the_scalar_form(q):
+    """Three packed fields of 47 MB and 64 MB of room: the first one fits, is given back, and trajectory and flow run as
+    on a lattice that cannot be paired; with room again they run in pairs."""
+    run(q, '''
+        gf = links((16, 16, 16, 32))
+        gm = q.GaugeMomentum(gf.geo)
+        gm.set_rand(q.RngState("memory"), 1.0)
+        ga, u, p = q.GaugeAction(2.13, -0.331), gf.copy(), gm.copy()
+        g32 = gf.copy(precision=q.F32)
+
+        def packed(f):
+            q.prof_reset()
+            q.prof_enable(True)
+            f()
+            q.synchronize()
+            q.prof_enable(False)
+            return q.prof_get("pair_pack")[1]
+
+        def trajectory():
+            u.__imatmul__(gf)
+            p.__imatmul__(gm)
+            q.run_hmc_evolve_pure_gauge(p, u, ga, None, 8, precision="mixed")
+
+        def flow():
+            g32.__imatmul__(gf)
+            q.gf_wilson_flow_step(g32, 0.02, c1=-0.331)
+
+        old = q.force_get_variant(q.F32, True)
+        q.force_set_variant(q.F32, True, 10)
+        trajectory(), flow()  # the scalar form, and the work fields that it needs
+        want = np.asarray(u), np.asarray(g32)
+        q.force_set_variant(q.F32, True, old)
+        q.release_field_pool()
+        with Filled(64 << 20):
+            free = torch.cuda.mem_get_info()[0]
+            assert packed(trajectory) == 0 and packed(flow) == 0
+            assert torch.cuda.mem_get_info()[0] == free
+            trajectory(), trajectory()  # recorded and replayed
+            got = [(np.asarray(u), np.asarray(g32))]
+        assert packed(trajectory) == 4 and packed(flow) == 2
+        trajectory(), trajectory()
+        got.append((np.asarray(u), np.asarray(g32)))
+        for links_, flowed in got:  # FP32: the tolerance of the paired form's own tests
+            assert np.abs(links_ - want[0]).max() < 2e-5 and np.abs(flowed - want[1]).max() < 2e-5
+    ''')
